@@ -237,7 +237,8 @@ void vfb_profile_reset(void *ctx);
  * tiles_log2 12, every resident CTA).  Results never depend on the shape. */
 #define VFB_TUNE_BANDS 16
 typedef struct {
-  uint8_t rows[VFB_TUNE_BANDS];         /* staged rows per tile: 1, 2, 4, .. 32 (above 16 acts as 16) */
+  uint8_t rows[VFB_TUNE_BANDS];         /* staged rows per tile: 1, 2, 4, .. 32 (at most 16, 8, 4, 2
+                                           for up to 16, 32, 64, 128 traces: more acts as that) */
   uint8_t tiles_log2[VFB_TUNE_BANDS];   /* tile count to reach by shorter tiles, log2 (1..40) */
   uint16_t blocks[VFB_TUNE_BANDS];      /* CTAs of the level's launch */
   float ms[VFB_TUNE_BANDS];             /* vfb_autotune: k_p1 time of the chosen shape summed

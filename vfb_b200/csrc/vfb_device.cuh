@@ -18,10 +18,8 @@ constexpr int kMaxSplits = 16;        // floor((32-1)/2)
 // binary level pairs; with unit costs, 1 + floor((k-1)/2)
 constexpr int kGroups = 64;
 constexpr int kTS = 128;              // stream rows per P1 tile (= threads per CTA)
-// Staged rows per P1 tile (maximum).  The shared memory of a tile holds kTS
-// stream rows and kTQ staged rows; 16 rather than 32 lets three CTAs share an
-// SM at 64 words per row instead of two (k_p1 of the large instance 40 ->
-// 34 ms), and 32 staged rows gained under 1% where the autotuner chose them.
+// Staged rows per P1 tile (maximum).  Only the staged rows are held in shared
+// memory (32 bytes per word, see QWord): 16 rows of 64 words are 32 KB.
 constexpr int kTQ = 16;
 constexpr int kTQDefault = 16;        // staged rows per P1 tile unless the tune table says otherwise
 constexpr int kP1TileTarget = 4096;   // shrink the staged height until a level has this many tiles
@@ -195,30 +193,38 @@ __device__ __forceinline__ uint64_t w_glob(uint64_t w, uint64_t lm) {
   return w & ~w_fin(~w & lm);
 }
 
-// l U r on one word: U_t = r_t | (l_t & U_{t+1}).  Reversing the bit order
-// turns the recurrence into a carry chain (generate = r, propagate = l), which
-// one 64-bit addition resolves; the carry out of bit 63 supplies the top bit.
-// Equal to the 6-step doubling of LTL_BS.cu:222-233 on every input.
-__device__ __forceinline__ uint64_t w_until(uint64_t l, uint64_t r) {
-  const uint64_t lr = __brevll(l), rr = __brevll(r);
-  const uint64_t a = lr | rr;
-  const uint64_t s = a + rr;
-  const uint64_t c = s ^ a ^ rr;
-  const uint64_t cout = (s < a) ? 1ULL : 0ULL;
-  return __brevll((c >> 1) | (cout << 63));
+// l U r on one word in the reversed bit order (lr, rr: the operands' words
+// reversed).  U_t = r_t | (l_t & U_{t+1}) is then a carry chain from low to
+// high bits (generate = r, propagate = l), which the addition s = (l|r) + r
+// resolves.  Bit by bit, with c the carry in: r = 1 gives U = 1; r = 0, l = 1
+// leaves s = ~c, and U is the carry in; r = l = 0 gives 0.  So U = r | (l & ~s):
+// neither the carries nor the carry out of the top bit are needed.
+__device__ __forceinline__ uint64_t until_rev(uint64_t lr, uint64_t rr) {
+  return rr | (lr & ~((lr | rr) + rr));
 }
 
-__device__ __forceinline__ uint64_t splitmix_fin(uint64_t x) {
-  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ULL;
-  x = (x ^ (x >> 27)) * 0x94d049bb133111ebULL;
-  return x ^ (x >> 31);
+// l U r on one word.  Equal to the 6-step doubling of LTL_BS.cu:222-233 on
+// every input.
+__device__ __forceinline__ uint64_t w_until(uint64_t l, uint64_t r) {
+  return __brevll(until_rev(__brevll(l), __brevll(r)));
 }
+
+// The splitmix64 finaliser of LTL_BS.cu:81-82 in two parts.  splitmix_mul is
+// everything after its first xor-shift (x: word ^ word >> 30) and before its
+// last one.  The last xor-shift is linear over XOR, so a fold of finalised
+// words applies it once to the fold instead of to every word (splitmix_end).
+__device__ __forceinline__ uint64_t splitmix_mul(uint64_t x) {
+  x *= 0xbf58476d1ce4e5b9ULL;
+  return (x ^ (x >> 27)) * 0x94d049bb133111ebULL;
+}
+__device__ __forceinline__ uint64_t splitmix_end(uint64_t x) { return x ^ (x >> 31); }
+__device__ __forceinline__ uint64_t splitmix_fin(uint64_t x) { return splitmix_end(splitmix_mul(x ^ (x >> 30))); }
 
 // ------------------------------------------------------------------ key state
 // Streaming accumulation of the 126-bit key of LTL_BS.cu:30-110 over the words
 // of one CS (word i of trace i, in trace order).
 struct KeyAcc {
-  uint64_t a0, a1;  // KEY_CONCAT/KEY_SAMPLED: bits 0..127; KEY_HASH: l, h
+  uint64_t a0, a1;  // KEY_CONCAT/KEY_SAMPLED: bits 0..127; KEY_HASH: l, h before splitmix_end
 };
 
 __device__ __forceinline__ void key_init(KeyAcc& k) { k.a0 = k.a1 = 0; }
@@ -234,7 +240,7 @@ template <int MODE>
 __device__ __forceinline__ void key_word(KeyAcc& k, uint64_t w, int i, int half, int off, int width,
                                          int stride, int L) {
   if (MODE == KEY_HASH) {
-    const uint64_t x = splitmix_fin(w);
+    const uint64_t x = splitmix_mul(w ^ (w >> 30));
     if (i < half) k.a1 ^= x; else k.a0 ^= x;   // a1 = h, a0 = l
   } else {
     uint64_t f = (MODE == KEY_SAMPLED) ? compress_stride(w, stride, L) : w;
@@ -252,8 +258,8 @@ __device__ __forceinline__ void key_word(KeyAcc& k, uint64_t w, int i, int half,
 template <int MODE>
 __device__ __forceinline__ void key_final(const KeyAcc& k, uint64_t& h, uint64_t& l) {
   if (MODE == KEY_HASH) {
-    h = k.a1;
-    l = k.a0;
+    h = splitmix_end(k.a1);
+    l = splitmix_end(k.a0);
   } else {
     const uint64_t lo = k.a0, hi = k.a1 & ((1ULL << 62) - 1ULL);   // 126 bits
     l = lo & ((1ULL << 63) - 1ULL);

@@ -98,9 +98,6 @@ struct Engine {
   // programmatic dependent launch between the kernels of a step (VFB_PDL=1):
   // measured 1-4% slower than plain stream order on every workload here
   bool use_pdl = false;
-  // P1 tiles staged by one bulk copy per operand block (VFB_P1_STAGING=bulk)
-  // instead of 8-byte asynchronous copies
-  bool p1_bulk = false;
   bool single_step = false;  // serving: one level per launch (admission between levels)
   bool use_coop = false;  // whole-GPU persistent cooperative solver (k_solve)
   int coop_grid = 0;
@@ -409,17 +406,13 @@ struct Engine {
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oe, k_emit, 256, 0) != cudaSuccess || oe < 1) oe = 1;
       emit_grid = sms * oe * 2;
     }
-    const int maxsmem = (kTS * (kMaxTraces + 1) + kTQ * kMaxTraces) * 8;
+    const int maxsmem = p1_smem_bytes(kMaxTraces);
     if (cudaFuncSetAttribute(k_p1, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsmem) != cudaSuccess)
       return VFB_DEVICE_ERROR;
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, k_p1) != cudaSuccess) return VFB_DEVICE_ERROR;
     if (cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsmem) != cudaSuccess)
       return VFB_DEVICE_ERROR;
-    if (cudaFuncSetAttribute(k_p1_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsmem) != cudaSuccess)
-      return VFB_DEVICE_ERROR;
-    const char* stg = std::getenv("VFB_P1_STAGING");
-    p1_bulk = stg && std::strcmp(stg, "bulk") == 0;
     const char* pdl_env = std::getenv("VFB_PDL");
     use_pdl = pdl_env && pdl_env[0] == '1';
     const char* env = std::getenv("VFB_NO_DEVICE_LOOP");
@@ -529,7 +522,7 @@ struct Engine {
       step_launch(false, k_advance, 1u, (unsigned)adv_threads, 0, dB, handle, built0, lp, mx);
       mark();
     }
-    step_launch(pdl && pre, p1_bulk ? k_p1_bulk : k_p1, (unsigned)p1_grid, (unsigned)kTS, (size_t)p1_smem, dB);
+    step_launch(pdl && pre, k_p1, (unsigned)p1_grid, (unsigned)kTS, (size_t)p1_smem, dB);
     mark();
     step_launch(pdl, k_table_scan_check, (unsigned)grid, 256u, 0, dB);
     mark();
@@ -1194,7 +1187,7 @@ struct Engine {
       }
       maxTP = std::max(maxTP, H[i].d.TP);
     }
-    const int p1_smem = (kTS * (maxTP + 1) + kTQ * maxTP) * 8;
+    const int p1_smem = p1_smem_bytes(maxTP);
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, p1_smem);
     p1_grid = sms * std::max(occ, 1);
@@ -1545,6 +1538,7 @@ struct Engine {
     uint64_t evictions = 0;       // requests evicted and queued again (memory held by the others)
     InstDev* h_inst = nullptr;    // pinned mirror of the slot records
     int p1_smem = 0;
+    int tp = 0;                   // row pitch of the most traces a request may have
     double budget_frac = 0.8;     // admission: projected bytes of all slots <= budget_frac * budget
     uint64_t request_bytes = 0;   // per-request cap (0: a quarter of the budget)
     uint64_t step_cands = 0;      // P1 candidates per request per step (0: whole levels)
@@ -1587,7 +1581,8 @@ struct Engine {
       return VFB_OOM;
     }
     const int tp = std::max(2, std::min(max_traces, (int)kMaxTraces) + (max_traces & 1));
-    sv.p1_smem = (kTS * (tp + 1) + kTQ * tp) * 8;
+    sv.tp = tp;
+    sv.p1_smem = p1_smem_bytes(tp);
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, sv.p1_smem);
     p1_grid = sms * std::max(occ, 1);
@@ -1735,7 +1730,7 @@ struct Engine {
       H = InstHost{};
       vfb_status s = prepare(p.in, H);
       const int tp = p.in.num_traces + (p.in.num_traces & 1);
-      if (s == VFB_OK && (kTS * (tp + 1) + kTQ * tp) * 8 > sv.p1_smem) s = VFB_LIMIT;
+      if (s == VFB_OK && tp > sv.tp) s = VFB_LIMIT;
       if (s == VFB_OK) {
         Caps c{4096, 1u << 14, 1u << 14, 1u << 13};
         c.rows = std::max<uint64_t>(c.rows, (uint64_t)H.d.A * 16);

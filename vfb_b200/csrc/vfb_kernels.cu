@@ -116,7 +116,7 @@ __device__ void plan_one(InstDev& I) {
     if (kind == 0) {
       const uint64_t st = (n[la] + kTS - 1) / kTS;
 #pragma unroll
-      for (int u = 0; u < 6; ++u) tl[u] += st;
+      for (int u = 0; u < 6; ++u) tl[u] += (st + (1ULL << u) - 1) >> u;
     } else {
       const bool qleft = (la == lb) || (n[la] <= n[lb]);
       const uint64_t nS = qleft ? n[lb] : n[la], nQ = qleft ? n[la] : n[lb];
@@ -204,13 +204,16 @@ __device__ void plan_one(InstDev& I) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) I.grp_base[q][u] = b4[u];
   }
-  // P1 tiling: kTS stream rows x tq staged rows per tile.  The staged height
+  // P1 tiling: kTS stream rows x tq staged rows per tile, or tq blocks of kTS
+  // rows of a unary group (about the same work).  The height
   // is the largest power of two within the band's bound whose tile count
   // reaches the band's target (small levels get shorter tiles so that they
   // still spread over every SM and end in a short last wave), else 1.  The
   // level's band of the tune table also sets the CTAs to launch.
   const int band = tune_band(g);
-  const int rows_cap = I.tune_rows[band] ? (I.tune_rows[band] < kTQ ? I.tune_rows[band] : kTQ) : kTQDefault;
+  const int rows_max = p1_rows_max(I.TP);
+  const int rows_want = I.tune_rows[band] ? I.tune_rows[band] : kTQDefault;
+  const int rows_cap = rows_want < rows_max ? rows_want : rows_max;
   const uint64_t target = I.tune_tiles[band] ? 1ULL << I.tune_tiles[band] : (uint64_t)kP1TileTarget;
   I.p1_blocks = I.tune_blocks[band];
   int lg = 0;
@@ -228,7 +231,7 @@ __device__ void plan_one(InstDev& I) {
       const int la = weighted ? I.grp_la[q] : u_la(q);
       const int lb = weighted ? I.grp_lb[q] : u_lb(q);
       if (kind == 0) {
-        acc += (n[la] + kTS - 1) / kTS;
+        acc += ((n[la] + kTS - 1) / kTS + (1ULL << lg) - 1) >> lg;
       } else {
         const bool qleft = (la == lb) || (n[la] <= n[lb]);
         const uint64_t nS = qleft ? n[lb] : n[la], nQ = qleft ? n[la] : n[lb];
@@ -349,51 +352,89 @@ __global__ void __launch_bounds__(1024) k_plan(BatchDev* Bp) {
 }
 
 // ======================================================================= P1
-// Bulk staging (BULK): a tile's stream rows and staged rows are each one
-// contiguous block of the level cache, copied into shared memory by one
-// cp.async.bulk apiece (issued by thread 0, completion counted by an
-// mbarrier in bytes).  The wait is bounded: a copy that has not landed after
-// about a second stops the instance with an error instead of hanging.
-constexpr long long kBulkWaitCycles = 2000000000LL;
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-               ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
-}
-
-// true when the barrier's phase `parity` completed within the bound
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity) {
-  const long long t0 = clock64();
-  for (;;) {
-    uint32_t done = 0;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 " selp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-    if (done) return true;
-    if (clock64() - t0 > kBulkWaitCycles) return false;
+// The instance's part of a tile's shared parameters (thread per trace), kept
+// while a CTA's consecutive tiles are of one instance.
+__device__ void p1_instance(const InstDev& I, TileSh& P) {
+  for (int t = threadIdx.x; t < P.TP; t += blockDim.x) {
+    const int L = t < P.T ? I.len[t] : 0;
+    P.len[t] = (uint8_t)L;
+    P.tr[t] = TraceSh{len_mask(L), t < P.T ? (uint32_t)pos_bit(P, t) : 0u, 0u};
+    P.off[t] = t < P.T ? I.off[t] : 0;
+    P.wid[t] = t < P.T ? I.width[t] : 0;
   }
-}
-
-template <bool BULK>
-__device__ void ph_p1(const BatchDev& B) {
-  extern __shared__ __align__(16) uint64_t smem[];
-  __shared__ TileSh P;
-  __shared__ unsigned long long s_red[3][kTS / 32];
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ int s_stop;
-  uint32_t phase = 0;
-  if (BULK) {
-    if (threadIdx.x == 0) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_addr(&s_bar)) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      s_stop = 0;
+  if (P.exact && threadIdx.x < 32) {
+    // masks over the key bits: a lane takes some traces, then XOR shuffles
+    KeyAcc full{0, 0}, last{0, 0}, first{0, 0}, want{0, 0};
+    for (int t = threadIdx.x; t < P.T; t += 32) {
+      const int L = I.len[t], off = I.off[t];
+      key_word<KEY_CONCAT>(full, len_mask(L), t, 0, off, L, 1, L);
+      key_word<KEY_CONCAT>(last, 1ULL << (L - 1), t, 0, off, L, 1, L);
+      key_word<KEY_CONCAT>(first, 1ULL, t, 0, off, L, 1, L);
+      key_word<KEY_CONCAT>(want, pos_bit(P, t), t, 0, off, L, 1, L);
     }
-    __syncthreads();
+    uint64_t v[8] = {full.a0, full.a1, last.a0, last.a1, first.a0, first.a1, want.a0, want.a1};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] ^= __shfl_xor_sync(0xffffffffu, v[j], o);
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        P.full[j] = v[j];
+        P.last[j] = v[2 + j];
+        P.first[j] = v[4 + j];
+        P.want[j] = v[6 + j];
+      }
+    }
   }
+  __syncthreads();
+}
+
+// The tile's staged rows into shared memory: their words (QWord) unless the
+// key bits alone settle the candidates, and their key bits (QKey) where keys
+// are bit fields.
+__device__ __forceinline__ void p1_stage(const InstDev& I, const TileSh& P, QWord* sQ, QKey* sK) {
+  const uint64_t* src = row_ptr(I, P.qi, P.q0);
+  const int T = P.T, TP = P.TP;
+  if (P.otf || !P.exact) {
+    // (nq rows of TP words: one block, the padding words zero)
+    const int dc = blockDim.x % TP;
+    int c = threadIdx.x % TP;
+    for (int x = threadIdx.x; x < P.nq * TP; x += blockDim.x) {
+      const uint64_t w = ld_row1(src + x);
+      sQ[x] = QWord{w, w >> 30, __brevll(w), P.tr[c].lab, 0u};
+      c += dc;
+      if (c >= TP) c -= TP;
+    }
+  }
+  if (P.mode != KEY_HASH && !P.otf) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < P.nq; r += blockDim.x >> 5) {
+      KeyAcc k;
+      key_init(k);
+      for (int t = lane; t < T; t += 32) {
+        const uint64_t w = ld_row1(src + (size_t)r * P.TP + t);
+        if (P.mode == KEY_SAMPLED) key_word<KEY_SAMPLED>(k, w, t, 0, P.off[t], P.wid[t], P.stride, P.len[t]);
+        else key_word<KEY_CONCAT>(k, w, t, 0, P.off[t], P.wid[t], P.stride, P.len[t]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        k.a0 ^= __shfl_xor_sync(0xffffffffu, k.a0, o);
+        k.a1 ^= __shfl_xor_sync(0xffffffffu, k.a1, o);
+      }
+      if (lane == 0) sK[r] = QKey{k.a0, k.a1, __brevll(k.a1), __brevll(k.a0)};
+    }
+  }
+}
+
+__device__ void ph_p1(const BatchDev& B) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ TileSh P;
+  __shared__ WarpIns s_ins[kTS / 32];
+  __shared__ unsigned long long s_red[3][kTS / 32];
   const unsigned long long total = B.p1_prefix[B.ninst];
+  InsState S{&s_ins[threadIdx.x >> 5], nullptr, 0, 0, 0, false};
+  int prev = -1;   // the instance whose part of P is loaded
   while (true) {
     if (threadIdx.x < 32) {
       // tile set-up by warp 0: the group boundaries are read one per lane and
@@ -446,7 +487,7 @@ __device__ void ph_p1(const BatchDev& B) {
           P.half = T / 2;
           P.stride = stride;
           P.mode = mode;
-          P.tq = tq;
+          P.exact = mode == KEY_CONCAT && __ldcg(&Ip->lensum) <= 126;
           P.pos[0] = pos0;
           P.pos[1] = pos1;
           // give up early once the table is known to be too small for this level
@@ -458,105 +499,131 @@ __device__ void ph_p1(const BatchDev& B) {
           // solution candidate found so far cannot change the result (every
           // candidate before it is still evaluated): they are skipped
           unsigned keep = 0xF;
+          int all = gmask;
           if (kind == 0) {
+            const uint64_t s0 = within * tq * kTS, blocks = (ni - s0 + kTS - 1) / kTS;
             P.si = i;
             P.nS = ni;
-            P.s0 = within * kTS;
+            P.s0 = s0;
+            P.nq = (int)(blocks < (uint64_t)tq ? blocks : (uint64_t)tq);
             if (may_skip && best != ~0ULL) {
               keep = 0;
 #pragma unroll
-              for (int u = 0; u < 4; ++u) keep |= (gb[u] + P.s0 <= best ? 1u : 0u) << u;
+              for (int u = 0; u < 4; ++u) keep |= (gb[u] + s0 <= best ? 1u : 0u) << u;
             }
           } else {
             const int qleft = (i == j) || (ni <= nj);
-            P.i = i;
-            P.j = j;
-            P.ni = ni;
-            P.nj = nj;
+            const uint64_t nS = qleft ? nj : ni, nQ = qleft ? ni : nj;
             P.qleft = qleft;
             P.si = qleft ? j : i;
             P.qi = qleft ? i : j;
-            P.nS = qleft ? nj : ni;
-            P.nQ = qleft ? ni : nj;
+            P.nS = nS;
+            P.nQ = nQ;
             uint64_t sq, qr;
             divmod64(within, qt, sq, qr);
-            P.s0 = sq * kTS;
-            P.q0 = qr * tq;
+            const uint64_t s0 = sq * kTS, q0 = qr * tq;
+            P.s0 = s0;
+            P.q0 = q0;
+            P.nq = (int)(nQ - q0 < (uint64_t)tq ? nQ - q0 : (uint64_t)tq);
+            // the U bits by the staged row's side (staged U stream, stream U
+            // staged) rather than by level
+            if (!qleft) {
+              all = (gmask & 3) | ((gmask & 4) << 1) | ((gmask & 8) >> 1);
+              const uint64_t x = gb[2];
+              gb[2] = gb[3];
+              gb[3] = x;
+            }
             if (may_skip && best != ~0ULL) {
-              const uint64_t amin = qleft ? P.q0 : P.s0, bmin = qleft ? P.s0 : P.q0;
-              const uint64_t ab = amin * nj + bmin;
+              const uint64_t qs = q0 * nS + s0, sm = s0 * nQ + q0, ab = qleft ? qs : sm;
               keep = (gb[0] + ab <= best ? 1u : 0u) | (gb[1] + ab <= best ? 2u : 0u) |
-                     (gb[2] + ab <= best ? 4u : 0u) | (gb[3] + bmin * ni + amin <= best ? 8u : 0u);
+                     (gb[2] + qs <= best ? 4u : 0u) | (gb[3] + sm <= best ? 8u : 0u);
             }
           }
-          P.mask = gmask & keep;
-          if (P.mask != gmask) *(volatile int*)&const_cast<InstDev*>(Ip)->p1_masked = 1;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) P.gb[u] = gb[u];
+          P.mask = all & keep;
+          if (P.mask != all) *(volatile int*)&const_cast<InstDev*>(Ip)->p1_masked = 1;
         }
       }
     }
     __syncthreads();
     if (P.tile >= total) break;
     InstDev& I = B.inst[P.inst];
-    for (int t = threadIdx.x; t < P.T; t += blockDim.x) {
-      P.len[t] = I.len[t];
-      P.off[t] = I.off[t];
-      P.wid[t] = I.width[t];
+    if (P.inst != prev) {
+      prev = P.inst;
+      p1_instance(I, P);
     }
-    // odd pitch for 8-byte copies (conflict-free row reads); the bulk copy
-    // keeps the rows' own pitch and rotates the word order instead
-    const int sp = BULK ? P.TP : P.TP + 1;
-    uint64_t* sS = smem;
-    uint64_t* sQ = smem + kTS * sp;
+    QKey* sK = reinterpret_cast<QKey*>(smem);
+    QWord* sQ = reinterpret_cast<QWord*>(smem) + kTQ;
     P1Count cnt{0, 0, ~0ULL};
     // a tile whose every operator is skipped has nothing to do
-    bool idle = P.skip || (!P.otf && P.mask == 0);
-    if (!idle) {
-      const int ns = (int)((P.nS - P.s0) < (uint64_t)kTS ? (P.nS - P.s0) : (uint64_t)kTS);
-      const int nq = P.kind == 1 ? (int)((P.nQ - P.q0) < (uint64_t)P.tq ? (P.nQ - P.q0) : (uint64_t)P.tq) : 0;
-      if (BULK) {
-        if (threadIdx.x == 0) {
-          // the previous tile's reads (generic proxy) come before these writes
-          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-          const uint32_t bs = (uint32_t)ns * P.TP * 8, bq = (uint32_t)nq * P.TP * 8;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-                       ::"r"(smem_addr(&s_bar)), "r"(bs + bq) : "memory");
-          bulk_copy(sS, row_ptr(I, P.si, P.s0), bs, &s_bar);
-          if (nq) bulk_copy(sQ, row_ptr(I, P.qi, P.q0), bq, &s_bar);
-        }
-        if (!bar_wait(&s_bar, phase)) {
-          *(volatile int*)&I.status = ST_ERROR;
-          s_stop = 1;
-        }
-        phase ^= 1u;
-      } else {
-        stage_rows(sS, sp, row_ptr(I, P.si, P.s0), ns, P.TP);
-        if (nq) stage_rows(sQ, P.TP, row_ptr(I, P.qi, P.q0), nq, P.TP);
-        stage_wait();
-      }
+    const bool idle = P.skip || (!P.otf && P.mask == 0);
+    S.list = !P.nolist;
+    S.tab = I.table;
+    S.mask = I.table_mask;
+    if (!idle && P.kind == 1) {
+      p1_stage(I, P, sQ, sK);
+      __syncthreads();
     }
-    __syncthreads();
-    if (BULK && s_stop) break;
+    const uint64_t* rows = row_ptr(I, P.si, 0);
     if (!idle && P.otf) {
-      p1_solutions<BULK>(I, P, sS, sp, sQ, cnt);
+      p1_solutions(P, rows, sQ, cnt);
     } else if (!idle) {
-      // binary tiles compute the operators up to the last one kept (& | laUlb lbUla)
-      const int keys = (P.mask & 8) ? 15 : (P.mask & 4) ? 7 : 3;
-      switch (P.mode) {
-        case KEY_HASH:
-          if (P.kind == 0 && P.mask == 1) p1_unary<KEY_HASH, BULK, 1>(I, P, sS, sp, cnt);
-          else if (P.kind == 0) p1_unary<KEY_HASH, BULK, 4>(I, P, sS, sp, cnt);
-          else p1_binary_keys<KEY_HASH, BULK>(keys, I, P, sS, sp, sQ, cnt);
-          break;
-        case KEY_SAMPLED:
-          if (P.kind == 0 && P.mask == 1) p1_unary<KEY_SAMPLED, BULK, 1>(I, P, sS, sp, cnt);
-          else if (P.kind == 0) p1_unary<KEY_SAMPLED, BULK, 4>(I, P, sS, sp, cnt);
-          else p1_binary_keys<KEY_SAMPLED, BULK>(keys, I, P, sS, sp, sQ, cnt);
-          break;
-        default:
-          if (P.kind == 0 && P.mask == 1) p1_unary<KEY_CONCAT, BULK, 1>(I, P, sS, sp, cnt);
-          else if (P.kind == 0) p1_unary<KEY_CONCAT, BULK, 4>(I, P, sS, sp, cnt);
-          else p1_binary_keys<KEY_CONCAT, BULK>(keys, I, P, sS, sp, sQ, cnt);
+      // a unary tile's rows, kTS a step, are one block of the level cache, read
+      // once: the next step's are on their way to the L2 during this one
+      auto ahead = [&](uint64_t at) {
+        if (threadIdx.x || at >= P.nS) return;
+        const uint64_t n = P.nS - at < (uint64_t)kTS ? P.nS - at : (uint64_t)kTS;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(rows + at * P.TP),
+                     "r"((unsigned)(n * P.TP * 8)));
+      };
+      if (P.kind == 0 || P.q0 == 0) ahead(P.s0);
+      uint64_t a = P.s0 + threadIdx.x;
+      const uint64_t* row = rows + (a < P.nS ? a : P.nS - 1) * P.TP;
+      KeyAcc sk{0, 0};
+      if (P.kind && P.mode != KEY_HASH)
+        sk = P.mode == KEY_SAMPLED ? row_bits<KEY_SAMPLED>(P, row) : row_bits<KEY_CONCAT>(P, row);
+      const bool one = P.mask == 1;
+      for (int q = 0; q < P.nq;) {
+        int done = 1;
+        Cands C;
+        C.ok = 0;
+        if (P.kind == 0) {
+          a = P.s0 + (uint64_t)q * kTS + threadIdx.x;
+          row = rows + (a < P.nS ? a : P.nS - 1) * P.TP;
+          if (q + 1 < P.nq) ahead(P.s0 + (uint64_t)(q + 1) * kTS);
+          switch (P.mode) {
+            case KEY_HASH: one ? p1_unary<KEY_HASH, 1>(P, row, a, C, cnt) : p1_unary<KEY_HASH, 4>(P, row, a, C, cnt); break;
+            case KEY_SAMPLED:
+              one ? p1_unary<KEY_SAMPLED, 1>(P, row, a, C, cnt) : p1_unary<KEY_SAMPLED, 4>(P, row, a, C, cnt);
+              break;
+            default: one ? p1_unary<KEY_CONCAT, 1>(P, row, a, C, cnt) : p1_unary<KEY_CONCAT, 4>(P, row, a, C, cnt);
+          }
+        } else {
+          switch (P.mode) {
+            case KEY_HASH: done = p1_pair<KEY_HASH>(P, row, sk, sQ, sK, q, C, cnt); break;
+            case KEY_SAMPLED: done = p1_pair<KEY_SAMPLED>(P, row, sk, sQ, sK, q, C, cnt); break;
+            default: done = p1_pair<KEY_CONCAT>(P, row, sk, sQ, sK, q, C, cnt);
+          }
+        }
+        q += done;
+        // two candidates at a time, so that the queue stays short (the drain's
+        // code is there once; the last drain of the tile empties the queue)
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) push_key(S, (C.ok >> j) & 1u, C.h[j], C.l[j], pay_of(P.k, C.g[j]));
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            C.h[j] = C.h[2 + j];
+            C.l[j] = C.l[2 + j];
+            C.g[j] = C.g[2 + j];
+          }
+          C.ok >>= 2;
+          drain_queue(I, S, q < P.nq || r == 0 ? 32 * kProbeKeys : 1, cnt);
+        }
       }
+      if (S.nl) flush_list(I, S, S.nl);
     }
     // per-tile counter flush: warp reductions, then one atomic per counter
     cnt.fresh = warp_sum(cnt.fresh);
@@ -589,24 +656,13 @@ __device__ void ph_p1(const BatchDev& B) {
   }
 }
 
-__global__ void __launch_bounds__(kTS) k_p1(BatchDev* Bp) {
+__global__ void __launch_bounds__(kTS, 4) k_p1(BatchDev* Bp) {
   step_entry();
   const BatchDev B = *Bp;
   if (blockIdx.x >= B.p1_prefix[B.ninst]) return;   // more CTAs than tiles: no ticket needed
   const unsigned long long cap = B.tickets[kTicketP1Blocks];
   if (cap && blockIdx.x >= cap) return;               // the tuned CTA count of this step
-  ph_p1<false>(B);
-}
-
-// k_p1 with bulk-copied tiles (VFB_P1_STAGING=bulk; measured against the
-// 8-byte copies of k_p1, see the design notes)
-__global__ void __launch_bounds__(kTS) k_p1_bulk(BatchDev* Bp) {
-  step_entry();
-  const BatchDev B = *Bp;
-  if (blockIdx.x >= B.p1_prefix[B.ninst]) return;
-  const unsigned long long cap = B.tickets[kTicketP1Blocks];
-  if (cap && blockIdx.x >= cap) return;
-  ph_p1<true>(B);
+  ph_p1(B);
 }
 
 // ============================================================== table scan
@@ -1386,7 +1442,7 @@ __global__ void __launch_bounds__(kTS) k_solve(BatchDev* Bp, unsigned int max_st
     if (!grid_sync(ctl, nb)) return;
     if (bid == 0 && threadIdx.x == 0) ph_plan_prefix(B);
     if (!grid_sync(ctl, nb)) return;
-    ph_p1<false>(B);
+    ph_p1(B);
     if (!grid_sync(ctl, nb)) return;
     ph_table_scan(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
@@ -1449,7 +1505,7 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
       cl.sync();
       if (rank == 0 && threadIdx.x == 0) ph_plan_prefix(B);
       cl.sync();
-      ph_p1<false>(B);
+      ph_p1(B);
       cl.sync();
       ph_table_scan(B, rank, csize);
       cl.sync();

@@ -23,6 +23,14 @@ constexpr int kEmitItem = 32;         // owners per k_emit work item on large le
                                       // their few owners still spread over many warps
 constexpr unsigned long long kEmitItemFrom = 1ULL << 18;   // owners from which items are kEmitItem
 
+// Staged rows of a P1 tile at most, and the dynamic shared memory of k_p1 for
+// rows of up to TP words: the staged rows' key bits and words (32 bytes each,
+// see QWord and QKey), at most 9 KB, so that the registers and not the shared
+// memory bound the CTAs of an SM.
+__host__ __device__ constexpr int p1_rows_max(int TP) { return TP > 64 ? 2 : TP > 32 ? 4 : TP > 16 ? 8 : kTQ; }
+__host__ __device__ constexpr int p1_smem_bytes(int TP) { return 32 * (kTQ + (TP > 16 ? 264 : kTQ * TP)); }
+static_assert(p1_rows_max(128) * 128 <= 264 && p1_rows_max(64) * 64 <= 264 && p1_rows_max(32) * 32 <= 264, "");
+
 // Global batch descriptor, resident in device memory so that buffer growth
 // never invalidates a captured launch sequence.
 struct BatchDev {
@@ -66,9 +74,6 @@ __global__ void k_emit(BatchDev* B);
 // launched in this order for every level.
 __global__ void k_plan(BatchDev* B);
 __global__ void k_p1(BatchDev* B);
-// k_p1 with each tile's operand blocks staged by cp.async.bulk (an option:
-// VFB_P1_STAGING=bulk).
-__global__ void k_p1_bulk(BatchDev* B);
 __global__ void k_table_scan(BatchDev* B);
 __global__ void k_chunk_count(BatchDev* B);
 __global__ void k_chunk_scan(BatchDev* B);

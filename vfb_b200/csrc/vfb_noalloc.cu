@@ -98,7 +98,7 @@ vfb_status scratch_base(int dev, unsigned char** out) {
       g_base[dev] = nullptr;
       return VFB_DEVICE_ERROR;
     }
-    const int smem = (kTS * (kMaxTraces + 1) + kTQ * kMaxTraces) * 8;
+    const int smem = p1_smem_bytes(kMaxTraces);
     if (cudaFuncSetAttribute(k_p1, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
       g_base[dev] = nullptr;
@@ -274,7 +274,7 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int g = sms * 8, gc = sms * 2;
-  const int p1_smem = (kTS * (d.TP + 1) + kTQ * d.TP) * 8;
+  const int p1_smem = p1_smem_bytes(d.TP);
   int occ = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, p1_smem);
   const int p1_grid = sms * (occ > 0 ? occ : 1);

@@ -361,150 +361,240 @@ __device__ inline void row_key(const InstDev& I, const uint64_t* row, uint64_t& 
 }
 
 // ======================================================================= P1
-// Shared per-tile parameters.
+// Shared per-tile parameters.  s: the stream operand (a row per thread), q:
+// the staged operand (up to kTQ rows, read by every thread).
+struct __align__(16) TraceSh {
+  uint64_t lm;     // length mask
+  uint32_t lab, pad;
+};
 struct TileSh {
   unsigned long long tile;
   int inst, grp, k, T, TP, half, stride, mode, skip;
-  int kind, mask;   // operand group: 0 unary / 1 binary; the operators it evaluates
+  int kind, mask;   // operand group: 0 unary (bits ~ X F G) / 1 binary (bits & | qUs sUq); the
+                    // operators it evaluates
   int otf;          // on-the-fly level: solution test only, nothing inserted
   int nolist;       // new slots are not listed (the table scan reads the whole table)
-  uint64_t s0, q0, nS, nQ, ni, nj;
-  int si, qi;   // levels of the stream / staged operand
-  int qleft;    // staged operand is the left operand of & | and of U(i->j)
-  int i, j, tq;
-  uint64_t pos[2];   // bit t: trace t is positive
+  int exact;        // every bit of every trace is in the key (KEY_CONCAT, no field cut)
+  uint64_t s0, q0, nS, nQ;
+  int si, qi, nq;   // levels of the stream / staged operand; staged rows of this tile
+  int qleft;        // the staged operand is the left operand of & | (its index is the major one)
+  uint64_t gb[4];   // candidate index of each operator of mask at rows (0, 0)
+  // ---- the instance's part (kept while consecutive tiles are of one instance)
+  uint64_t pos[2];  // bit t: trace t is positive
+  TraceSh tr[kMaxTraces];    // (the padding word's trace: all zero)
   uint8_t len[kMaxTraces], off[kMaxTraces], wid[kMaxTraces];
+  // exact keys: masks over the 126 key bits: every bit; the last step of
+  // each trace; its first step; the labels at the first steps
+  unsigned long long full[2], last[2], first[2], want[2];
 };
 
-// Copy nrows consecutive rows (pitch TP words) into shared memory with pitch
-// sp, one 8-byte asynchronous copy per word (cp.async: no registers held, every
-// copy of the tile in flight at once); stage_wait() completes them.  Rows
-// with an odd pitch are only 8-byte aligned, hence 8-byte copies.
-__device__ __forceinline__ void stage_rows(uint64_t* dst, int sp, const uint64_t* src, int nrows, int TP) {
-  const int n = nrows * TP;
-  const int dr = blockDim.x / TP, dc = blockDim.x - dr * TP;
-  int r = threadIdx.x / TP, c = threadIdx.x - r * TP;
-  for (int w = threadIdx.x; w < n; w += blockDim.x) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(dst + r * sp + c);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(src + w) : "memory");
-    r += dr;
-    c += dc;
-    if (c >= TP) { c -= TP; ++r; }
-  }
-}
-
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+// One staged word: the word, the word >> 30 (first xor-shift of the hash), its
+// bits reversed (U), and the trace's label.
+struct __align__(16) QWord {
+  uint64_t w, sh, rev;
+  uint32_t lab, pad;
+};
+// One staged row of keys that are bit fields: the key's bits, and reversed.
+struct __align__(16) QKey {
+  uint64_t k0, k1, r0, r1;
+};
+constexpr int kQWordBytes = 32;
+static_assert(sizeof(QWord) == kQWordBytes && sizeof(QKey) == kQWordBytes, "");
 
 struct P1Count {
   unsigned long long fresh, fail, sol;   // keys inserted, probe failures, min solution candidate
 };
 
-// Insert N keys of one thread: all home-slot loads are issued first, then the
-// keys are resolved one by one.  bad[j] == 0 marks a candidate whose step-0
-// bits match every trace's label (a solution candidate).
-template <int N>
-__device__ __forceinline__ void insert_group(InstDev& I, unsigned live, int k, const uint64_t* h,
-                                             const uint64_t* l, const uint64_t* g, const uint32_t* bad,
-                                             P1Count& cnt, unsigned valid, bool list) {
-  Slot* tab = I.table;
-  const uint64_t mask = I.table_mask;
-  uint64_t idx[N];
-  Key128 cur[N];
+__device__ __forceinline__ uint64_t ld_row1(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p));
+  return v;
+}
+// Two words of a row (rows start on 16-byte boundaries).
+__device__ __forceinline__ void ld_row2(const uint64_t* p, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.global.v2.u64 {%0, %1}, [%2];\n" : "=l"(a), "=l"(b) : "l"(p));
+}
+
+// body(t, a, b) over the words t = 0, 2, .. TP-2 and t+1 of a row in global
+// memory (padding words are zero), snap() before word mid (even).  Every lane
+// reads its own row; the next four words are loaded before the current four
+// are used.  Measured on the large instance (k_p1 per solve, 20.3 ms): rows
+// copied into shared memory eight words ahead, coalesced, 24.1 ms (a tenth
+// more instructions); 32-byte loads where the pitch allows 21.5 ms; loads six
+// or eight words ahead 22.0-22.7 ms.
+template <typename F, typename G>
+__device__ __forceinline__ void row_pass(const uint64_t* row, int TP, int mid, F&& body, G&& snap) {
+  auto fetch = [&](int t, uint64_t (&x)[4]) {   // t a multiple of 4 below TP
+    ld_row2(row + t, x[0], x[1]);
+    ld_row2(row + (t + 2 < TP ? t + 2 : t), x[2], x[3]);
+  };
+  uint64_t v[4];
+  fetch(0, v);
+#pragma unroll 1
+  for (int t = 0; t < TP; t += 4) {
+    uint64_t n[4];
+    fetch(t + 4 < TP ? t + 4 : t, n);
+    const int end = t + 4 < TP ? t + 4 : TP;
+#pragma unroll 1
+    for (int p = t; p < end; p += 2) {
+      if (p == mid) snap();
+      body(p, v[0], v[1]);
+      v[0] = v[2];
+      v[1] = v[3];
+    }
 #pragma unroll
-  for (int j = 0; j < N; ++j) idx[j] = slot_hash(h[j], l[j]) & mask;
-#pragma unroll
-  for (int j = 0; j < N; ++j) cur[j] = ld_key(tab + idx[j]);
-  uint64_t fresh[N];
-  int nf = 0;
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    if (!((valid >> j) & 1u)) continue;
-    int isnew = 0;
-    const int r = insert_min(tab, mask, idx[j], cur[j], h[j], l[j], pay_of(k, g[j]), isnew);
-    if (r < 0) ++cnt.fail;
-    if (isnew) fresh[nf++] = idx[j];
-    if (!bad[j] && g[j] < cnt.sol) cnt.sol = g[j];
+    for (int u = 0; u < 4; ++u) v[u] = n[u];
   }
-  cnt.fresh += nf;
-  if (!list) return;   // (warp-uniform)
-  // list the slots of the keys this warp inserted: one atomic per warp, the
-  // per-lane offsets from three ballots of the lane's count (0..4)
+}
+
+// ------------------------------------------------ P1's inserts, a warp at a time
+// Every candidate's key goes through the warp's queue in shared memory, and
+// the queue is worked off kProbeKeys keys per lane at a time: their slots'
+// loads, then the CAS of the empty ones, are in flight together.  A key whose
+// slot holds another key goes back into the queue for the next slot (linear
+// probing), so no lane idles while another follows a chain.  (Resolving every
+// thread's four keys in turn, each with its own chain, made the warp wait for
+// its longest chain four times over: 23.5 against 20.3 ms of k_p1 on the large
+// instance.)  The probe code is there once, whatever the operators computed: a
+// copy per operator set ran out of instruction cache (34 ms).
+struct __align__(16) Pend {
+  uint64_t h, l, pay;
+  uint64_t at;   // slot to try next; probes made << kProbeShift
+};
+constexpr int kProbeShift = 48;
+constexpr int kProbeKeys = 2;                          // keys per lane and step
+constexpr int kPushKeys = 2;                           // keys per lane queued between two drains
+constexpr int kPendCap = 32 * (kProbeKeys + kPushKeys);
+constexpr int kNewCap = 64;                            // listed slots: below 32, plus 32
+struct WarpIns {
+  Pend pend[kPendCap];
+  uint64_t fresh[kNewCap];   // slots of new keys, written to the level's list 32 at a time
+};
+// The warp's side of the queue (every lane holds the same counts).
+struct InsState {
+  WarpIns* w;
+  Slot* tab;
+  uint64_t mask;   // of the tile's instance
+  int np, nl;
+  bool list;
+};
+
+// Key and payload of a slot, from L2.
+struct SlotVal {
+  Key128 key;
+  unsigned long long pay;
+};
+__device__ __forceinline__ SlotVal ld_slot(const Slot* s) {
+  const ulonglong2 k = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+  return SlotVal{Key128{k.x, k.y}, __ldcg(&s->pay)};
+}
+
+// CAS (empty -> key) of a slot where p; else {0, 0}.  Predicated rather than
+// branched around, so that several are issued before the first is awaited.
+__device__ __forceinline__ Key128 cas_key(bool p, Slot* s, uint64_t h, uint64_t l) {
+  Key128 old;
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b128 e, n, o;\n setp.ne.u32 p, %2, 0;\n mov.b128 e, {%6, %6};\n"
+      " mov.b128 n, {%4, %5};\n mov.b128 o, {%7, %7};\n @p atom.relaxed.gpu.global.cas.b128 o, [%3], e, n;\n"
+      " mov.b128 {%0, %1}, o;\n}\n"
+      : "=l"(old.h), "=l"(old.l)
+      : "r"((unsigned)p), "l"(s), "l"(h), "l"(l), "l"((uint64_t)kEmpty), "l"(0ULL)
+      : "memory");
+  return old;
+}
+__device__ __forceinline__ void lower_pay(bool p, Slot* s, unsigned long long pay) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p red.relaxed.gpu.global.min.u64 [%1], %2;\n}\n"
+               ::"r"((unsigned)p), "l"(&s->pay), "l"(pay) : "memory");
+}
+
+// Writes n (at most 32) listed slots to the level's list; the rest move up.
+__device__ __forceinline__ void flush_list(InstDev& I, InsState& S, int n) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(&I.n_newlist, (unsigned long long)n);
+  const uint64_t v = S.w->fresh[lane], r = S.w->fresh[32 + lane];
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (lane < n && base + lane < I.tent_cap) I.wins[base + lane] = v;
+  __syncwarp();
+  if (n == 32) S.w->fresh[lane] = r;
+  __syncwarp();
+  S.nl -= n;
+}
+
+// Queues this lane's key (ok; whole warps call this), to start at its home slot.
+__device__ __forceinline__ void push_key(InsState& S, bool ok, uint64_t h, uint64_t l, unsigned long long pay) {
+  const unsigned m = __ballot_sync(0xffffffffu, ok);
+  if (ok) {
+    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+    S.w->pend[S.np + __popc(m & lt)] = Pend{h, l, pay, slot_hash(h, l) & S.mask};
+  }
+  S.np += __popc(m);
+}
+
+// Works the queue off until fewer than `keep` keys are left.
+__device__ __forceinline__ void drain_queue(InstDev& I, InsState& S, int keep, P1Count& cnt) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  const unsigned b0 = __ballot_sync(live, nf & 1), b1 = __ballot_sync(live, nf & 2),
-                 b2 = __ballot_sync(live, nf & 4);
-  const unsigned pre = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
-  const unsigned tot = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-  const int leader = __ffs(live) - 1;
-  unsigned long long base = 0;
-  if (lane == leader && tot) base = atomicAdd(&I.n_newlist, (unsigned long long)tot);
-  base = __shfl_sync(live, base, leader);
-  for (int r = 0; r < nf; ++r) {
-    const unsigned long long pos = base + pre + r;
-    if (pos < I.tent_cap) I.wins[pos] = fresh[r];
+  while (S.np >= keep) {
+    __syncwarp();
+    const int take = S.np < 32 * kProbeKeys ? S.np : 32 * kProbeKeys;
+    S.np -= take;
+    Pend k[kProbeKeys];
+    SlotVal cur[kProbeKeys];
+    Slot* sl[kProbeKeys];
+#pragma unroll
+    for (int j = 0; j < kProbeKeys; ++j) {
+      const int e = lane + 32 * j;
+      k[j] = S.w->pend[S.np + (e < take ? e : 0)];
+      sl[j] = S.tab + (k[j].at & S.mask);
+      cur[j] = SlotVal{Key128{k[j].h, k[j].l}, 0};   // (no key: reads as one that needs nothing)
+      if (e < take) cur[j] = ld_slot(sl[j]);
+    }
+    __syncwarp();   // (every entry is read before a push overwrites it)
+    // A real key never has a half equal to ~0 (normalised away), so a ~0 half
+    // is either an empty slot or a key being published: resolve with the CAS.
+    Key128 old[kProbeKeys];
+    unsigned tried = 0;
+#pragma unroll
+    for (int j = 0; j < kProbeKeys; ++j) {
+      const bool e = cur[j].key.h == kEmpty || cur[j].key.l == kEmpty;
+      tried |= (unsigned)e << j;
+      old[j] = cas_key(e, sl[j], k[j].h, k[j].l);
+    }
+#pragma unroll
+    for (int j = 0; j < kProbeKeys; ++j) {
+      const bool e = (tried >> j) & 1u;
+      const Key128 now = e ? old[j] : cur[j].key;
+      const bool fresh = e && now.h == kEmpty && now.l == kEmpty;   // this lane published the key
+      const bool same = now.h == k[j].h && now.l == k[j].l;
+      // (the payload of a key just published, here or by another lane, is
+      // lowered without a read; of one that was there only if this comes first)
+      lower_pay(fresh || (same && (e || cur[j].pay > k[j].pay)), sl[j], k[j].pay);
+      cnt.fresh += fresh;
+      if (S.list) {
+        const unsigned m = __ballot_sync(0xffffffffu, fresh);
+        if (m) {
+          if (fresh) S.w->fresh[S.nl + __popc(m & lt)] = k[j].at & S.mask;
+          S.nl += __popc(m);
+          if (S.nl >= 32) flush_list(I, S, 32);
+        }
+      }
+      const uint64_t probes = (k[j].at >> kProbeShift) + 1;
+      const bool more = !fresh && !same, lost = more && probes >= (uint64_t)kMaxProbes;
+      cnt.fail += lost;
+      const unsigned m = __ballot_sync(0xffffffffu, more && !lost);
+      if (m) {
+        if (more && !lost)
+          S.w->pend[S.np + __popc(m & lt)] = Pend{k[j].h, k[j].l, k[j].pay, ((k[j].at + 1) & S.mask) | (probes << kProbeShift)};
+        S.np += __popc(m);
+      }
+    }
   }
 }
 
 __device__ __forceinline__ uint64_t pos_bit(const TileSh& P, int t) {
   return (P.pos[t >> 6] >> (t & 63)) & 1ULL;
-}
-
-// Compile-time half of a trace index: HASH keys fold traces t < T/2 into h,
-// the others into l (LTL_BS.cu:30-110), so the P1 loops run the two halves
-// as separate loops and pick the accumulator statically.
-template <bool HI>
-struct Half {
-  static constexpr bool hi = HI;
-  static constexpr bool fixed = true;
-};
-// The half decided at run time (rotated word order of the bulk-staged tiles).
-struct HalfRt {
-  bool hi;
-  static constexpr bool fixed = false;
-};
-
-template <int MODE, bool HI>
-__device__ __forceinline__ void key_word_h(KeyAcc& k, uint64_t w, int t, int off, int width, int stride, int L) {
-  if (MODE == KEY_HASH) {
-    const uint64_t x = splitmix_fin(w);
-    if (HI) k.a1 ^= x; else k.a0 ^= x;
-  } else {
-    key_word<MODE>(k, w, t, 0, off, width, stride, L);
-  }
-}
-
-template <int MODE, typename H>
-__device__ __forceinline__ void key_word_any(KeyAcc& k, uint64_t w, int t, H half, int off, int width, int stride,
-                                             int L) {
-  if constexpr (H::fixed) {
-    key_word_h<MODE, H::hi>(k, w, t, off, width, stride, L);
-  } else if (MODE == KEY_HASH) {
-    const uint64_t x = splitmix_fin(w), m = half.hi ? ~0ULL : 0ULL;
-    k.a1 ^= x & m;
-    k.a0 ^= x & ~m;
-  } else {
-    key_word<MODE>(k, w, t, 0, off, width, stride, L);
-  }
-}
-
-// The trace words of a tile row in the order a thread visits them.  Copied
-// rows (odd pitch): 0..T-1, the words below T/2 first (the hash folds the two
-// halves into different words, chosen at compile time).  Bulk-staged rows
-// (pitch TP, even): lane l starts at word l mod T and wraps, so the 16 lanes
-// of a shared-memory wavefront read 16 different banks; the half is then
-// decided per word.
-template <bool BULK, typename F>
-__device__ __forceinline__ void p1_words(const TileSh& P, F&& body) {
-  if (!BULK) {
-    for (int t = 0; t < P.half; ++t) body(t, Half<true>{});
-    for (int t = P.half; t < P.T; ++t) body(t, Half<false>{});
-  } else {
-    int t = (threadIdx.x & 31) % P.T;
-    for (int i = 0; i < P.T; ++i) {
-      body(t, HalfRt{t < P.half});
-      if (++t == P.T) t = 0;
-    }
-  }
 }
 
 // Solution test accumulators: only bit 0 (step 0) of a word is compared
@@ -545,167 +635,374 @@ __device__ __forceinline__ void record_unary(InstDev& I, int k, uint64_t row, un
     if (!((miss >> o) & 1u)) atomicMax(&I.uhit[k][o], v);
 }
 
-// BULK: rows staged by one bulk copy at the even pitch TP (rotated word
-// order), else by 8-byte copies at the odd pitch TP + 1.
+// ---- keys that hold every bit of every trace (at most 126 bits)
+// The key of a candidate follows from its operands' keys: the operators act on
+// all traces at once, the trace fields side by side in 128 bits.  A step must
+// not reach into the next field: ~ and X mask it off, and U (a carry chain in
+// the reversed order, see until_rev) clears the left operand at each trace's
+// last step, where U = r whatever the carry.
+struct Bits128 {
+  uint64_t a, b;   // bits 0-63, 64-127
+};
+__device__ __forceinline__ Bits128 rev128(Bits128 x) { return Bits128{__brevll(x.b), __brevll(x.a)}; }
+// ln: left operand reversed with the last steps cleared; rr: right operand reversed
+__device__ __forceinline__ Bits128 until_exact(Bits128 ln, Bits128 rr) {
+  const uint64_t x = ln.a | rr.a, y = ln.b | rr.b;
+  uint64_t s, t;
+  asm("add.cc.u64 %0, %2, %3;\n\taddc.u64 %1, %4, %5;\n" : "=&l"(s), "=l"(t) : "l"(x), "l"(rr.a), "l"(y), "l"(rr.b));
+  return rev128(Bits128{rr.a | (ln.a & ~s), rr.b | (ln.b & ~t)});
+}
+__device__ __forceinline__ void exact_key(const TileSh& P, Bits128 x, uint64_t& h, uint64_t& l, uint32_t& bad) {
+  key_final<KEY_CONCAT>(KeyAcc{x.a, x.b}, h, l);
+  bad = (((x.a ^ P.want[0]) & P.first[0]) | ((x.b ^ P.want[1]) & P.first[1])) != 0 ? 1u : 0u;
+}
+
+// Up to four candidates of a lane, waiting to be queued.
+struct Cands {
+  uint64_t h[4], l[4], g[4];
+  unsigned ok;    // bit j: candidate j is there
+};
+
+// Key bits of a row, one thread per row (bit-field modes).
+template <int MODE>
+__device__ __forceinline__ KeyAcc row_bits(const TileSh& P, const uint64_t* row) {
+  KeyAcc k;
+  key_init(k);
+  auto word = [&](int t, uint64_t w) { key_word<MODE>(k, w, t, 0, P.off[t], P.wid[t], P.stride, P.len[t]); };
+  row_pass(row, P.TP, -1, [&](int t, uint64_t a, uint64_t b) {
+    word(t, a);
+    word(t + 1, b);
+  }, [] {});
+  return k;
+}
+
+// Candidate j of a lane (ok: it is one).  bad: bit 0 is clear when its step-0
+// bits match every trace's label.
+__device__ __forceinline__ void take_cand(Cands& C, int j, bool ok, uint64_t g, uint32_t bad, P1Count& cnt) {
+  C.g[j] = g;
+  C.ok |= (unsigned)ok << j;
+  if (ok && !(bad & 1u) && g < cnt.sol) cnt.sol = g;
+}
+
+// ---- unary tiles: a row per thread (row a of the level), its ~ X F G candidates
 // NU: the operators computed, ~ alone (1: every other one lies past the
 // level's first solution) or ~ X F G (4; the inserted ones are P.mask).
-template <int MODE, bool BULK, int NU>
-__device__ inline void p1_unary(InstDev& I, const TileSh& P, const uint64_t* sS, int sp, P1Count& cnt) {
-  const uint64_t a = P.s0 + threadIdx.x;
-  const unsigned live = __ballot_sync(0xffffffffu, a < P.nS);
-  if (a >= P.nS) return;
-  const uint64_t* srow = sS + threadIdx.x * sp;
-  KeyAcc k0, k1, k2, k3;
-  key_init(k0);
-  if (NU == 4) { key_init(k1); key_init(k2); key_init(k3); }
+template <int MODE, int NU>
+__device__ __forceinline__ void p1_unary(const TileSh& P, const uint64_t* row, uint64_t a, Cands& C, P1Count& cnt) {
   uint32_t bad[4] = {0, 0, 0, 0};
-  auto body = [&](int t, auto half) {
-    const uint64_t w = srow[t];
-    const int L = P.len[t], off = P.off[t], wd = P.wid[t];
-    const uint64_t lm = len_mask(L);
-    const uint32_t pb = (uint32_t)pos_bit(P, t);
-    const uint64_t w0 = ~w & lm;
-    bad[0] |= lo32(w0) ^ pb;
-    key_word_any<MODE>(k0, w0, t, half, off, wd, P.stride, L);
+  if (MODE == KEY_CONCAT && P.exact) {
+    const KeyAcc k = row_bits<KEY_CONCAT>(P, row);
+    const Bits128 w{k.a0, k.a1}, n{~w.a & P.full[0], ~w.b & P.full[1]};
+    exact_key(P, n, C.h[0], C.l[0], bad[0]);
     if (NU == 4) {
-      const uint64_t w1 = w >> 1, w2 = w_fin(w), w3 = w_glob(w, lm);
-      bad[1] |= lo32(w1) ^ pb;
-      bad[2] |= lo32(w2) ^ pb;
-      bad[3] |= lo32(w3) ^ pb;
-      key_word_any<MODE>(k1, w1, t, half, off, wd, P.stride, L);
-      key_word_any<MODE>(k2, w2, t, half, off, wd, P.stride, L);
-      key_word_any<MODE>(k3, w3, t, half, off, wd, P.stride, L);
+      exact_key(P, Bits128{((w.a >> 1) | (w.b << 63)) & ~P.last[0], (w.b >> 1) & ~P.last[1]}, C.h[1], C.l[1], bad[1]);
+      // F w = true U w, G w = ~F~w
+      const Bits128 p = rev128(Bits128{P.full[0] & ~P.last[0], P.full[1] & ~P.last[1]});
+      exact_key(P, until_exact(p, rev128(w)), C.h[2], C.l[2], bad[2]);
+      const Bits128 fn = until_exact(p, rev128(n));
+      exact_key(P, Bits128{~fn.a & P.full[0], ~fn.b & P.full[1]}, C.h[3], C.l[3], bad[3]);
     }
-  };
-  p1_words<BULK>(P, body);
-  uint64_t h[4], l[4], g[4];
-  key_final<MODE>(k0, h[0], l[0]);
-  g[0] = I.base_not + a;
-  if (NU == 4) {
-    key_final<MODE>(k1, h[1], l[1]);
-    key_final<MODE>(k2, h[2], l[2]);
-    key_final<MODE>(k3, h[3], l[3]);
-    g[1] = I.base_x + a;
-    g[2] = I.base_f + a;
-    g[3] = I.base_g + a;
-  }
+  } else if (MODE == KEY_HASH) {
+    uint64_t acc[NU], hi[NU];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) bad[j] &= 1u;
-  insert_group<NU>(I, live, P.k, h, l, g, bad, cnt, (unsigned)P.mask, !P.nolist);
-}
-
-// KEYS: the operators computed, a prefix of (&, |, laUlb, lbUla) as bits
-// 3, 7, 15; the inserted ones are P.mask within it.
-template <int MODE, int KEYS, bool BULK>
-__device__ inline void p1_binary(InstDev& I, const TileSh& P, const uint64_t* sS, int sp, const uint64_t* sQ,
-                          P1Count& cnt) {
-  constexpr bool kO = (KEYS & 2) != 0, kU = (KEYS & 4) != 0, kV = (KEYS & 8) != 0;
-  constexpr int N = 1 + (kO ? 1 : 0) + (kU ? 1 : 0) + (kV ? 1 : 0);
-  const uint64_t s = P.s0 + threadIdx.x;
-  const unsigned live = __ballot_sync(0xffffffffu, s < P.nS);
-  if (s >= P.nS) return;
-  const uint64_t* srow = sS + threadIdx.x * sp;
-  const int nq = (int)((P.nQ - P.q0) < (uint64_t)P.tq ? (P.nQ - P.q0) : (uint64_t)P.tq);
-  for (int q = 0; q < nq; ++q) {
-    const uint64_t* qrow = sQ + q * P.TP;
-    KeyAcc kA, kOr, kUn, kVn;
-    key_init(kA);
-    if (kO) key_init(kOr);
-    if (kU) key_init(kUn);
-    if (kV) key_init(kVn);
-    uint32_t bad[4] = {0, 0, 0, 0};
-    auto body = [&](int t, auto half) {
-      const uint64_t qw = qrow[t], sw = srow[t];
-      const uint64_t la = P.qleft ? qw : sw, lb = P.qleft ? sw : qw;
-      const int L = P.len[t], off = P.off[t], wd = P.wid[t];
-      const uint32_t pb = (uint32_t)pos_bit(P, t);
-      const uint64_t wa = la & lb;
-      bad[0] |= lo32(wa) ^ pb;
-      key_word_any<MODE>(kA, wa, t, half, off, wd, P.stride, L);
-      if (kO) {
-        const uint64_t wo = la | lb;
-        bad[1] |= lo32(wo) ^ pb;
-        key_word_any<MODE>(kOr, wo, t, half, off, wd, P.stride, L);
-      }
-      if (kU) {
-        const uint64_t wu = w_until(la, lb);
-        bad[2] |= lo32(wu) ^ pb;
-        key_word_any<MODE>(kUn, wu, t, half, off, wd, P.stride, L);
-      }
-      if (kV) {
-        const uint64_t wv = w_until(lb, la);
-        bad[3] |= lo32(wv) ^ pb;
-        key_word_any<MODE>(kVn, wv, t, half, off, wd, P.stride, L);
+    for (int j = 0; j < NU; ++j) acc[j] = hi[j] = 0;
+    auto fold = [&](int j, uint64_t w, uint32_t lab) {
+      bad[j] |= lo32(w) ^ lab;
+      acc[j] ^= splitmix_mul(w ^ (w >> 30));
+    };
+    auto word = [&](int t, uint64_t w) {
+      const TraceSh x = P.tr[t];
+      const uint64_t n = ~w & x.lm;
+      fold(0, n, x.lab);
+      if (NU == 4) {
+        fold(1 % NU, w >> 1, x.lab);
+        fold(2 % NU, w_fin(w), x.lab);
+        fold(3 % NU, w & ~w_fin(n), x.lab);
       }
     };
-    p1_words<BULK>(P, body);
-    const uint64_t a = P.qleft ? P.q0 + q : s;     // index in level i
-    const uint64_t b = P.qleft ? s : P.q0 + q;     // index in level j
-    const uint64_t ab = a * P.nj + b;
-    uint64_t h[4], l[4], g[4];
-    key_final<MODE>(kA, h[0], l[0]);
-    g[0] = I.base_and[P.i] + ab;
-    if (kO) { key_final<MODE>(kOr, h[1], l[1]); g[1] = I.base_or[P.i] + ab; }
-    if (kU) { key_final<MODE>(kUn, h[2], l[2]); g[2] = I.base_u[P.i] + ab; }
-    if (kV) { key_final<MODE>(kVn, h[3], l[3]); g[3] = I.base_u[P.j] + b * P.ni + a; }
+    auto snap = [&] {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) bad[j] &= 1u;
-    insert_group<N>(I, live, P.k, h, l, g, bad, cnt, (unsigned)P.mask & (unsigned)KEYS, !P.nolist);
+      for (int j = 0; j < NU; ++j) hi[j] = acc[j];
+    };
+    row_pass(row, P.TP, P.half & ~1, [&](int t, uint64_t x, uint64_t y) {
+      word(t, x);
+      word(t + 1, y);
+    }, snap);
+    // the words below T/2 fold into h, the others into l: hi is the fold up
+    // to the even word below, an odd T/2's last word is folded in once more
+    uint64_t all[NU];
+#pragma unroll
+    for (int j = 0; j < NU; ++j) {
+      all[j] = acc[j];
+      acc[j] = 0;
+    }
+    if (P.half & 1) word(P.half - 1, ld_row1(row + P.half - 1));
+#pragma unroll
+    for (int j = 0; j < NU; ++j) key_final<KEY_HASH>(KeyAcc{all[j] ^ hi[j] ^ acc[j], hi[j] ^ acc[j]}, C.h[j], C.l[j]);
+  } else {
+    KeyAcc k[NU];
+#pragma unroll
+    for (int j = 0; j < NU; ++j) key_init(k[j]);
+    auto word = [&](int t, uint64_t w) {
+      const TraceSh x = P.tr[t];
+      const int L = P.len[t], off = P.off[t], wd = P.wid[t];
+      auto put = [&](int j, uint64_t v) {
+        bad[j] |= lo32(v) ^ x.lab;
+        key_word<MODE>(k[j], v, t, 0, off, wd, P.stride, L);
+      };
+      put(0, ~w & x.lm);
+      if (NU == 4) {
+        put(1 % NU, w >> 1);
+        put(2 % NU, w_fin(w));
+        put(3 % NU, w_glob(w, x.lm));
+      }
+    };
+    row_pass(row, P.TP, -1, [&](int t, uint64_t x, uint64_t y) {
+      word(t, x);
+      word(t + 1, y);
+    }, [] {});
+#pragma unroll
+    for (int j = 0; j < NU; ++j) key_final<MODE>(k[j], C.h[j], C.l[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NU; ++j) take_cand(C, j, a < P.nS && ((P.mask >> j) & 1), P.gb[j] + a, bad[j], cnt);
+}
+
+// ---- binary tiles: a stream row per thread against the staged rows
+// KEYS: the operators computed, among & (1), | (2), staged U stream (4),
+// stream U staged (8); the inserted ones are P.mask within it.
+template <int K>
+struct Keys {
+  static constexpr int value = K;
+};
+__host__ __device__ constexpr int key_count(int keys) {
+  return (keys & 1) + ((keys >> 1) & 1) + ((keys >> 2) & 1) + ((keys >> 3) & 1);
+}
+
+// Candidates j0.. of one pair (in the order of the bits of KEYS).
+template <int KEYS>
+__device__ __forceinline__ void take_pair(const TileSh& P, uint64_t q, uint64_t s, int j, const uint32_t* bad,
+                                          Cands& C, P1Count& cnt) {
+  const uint64_t qs = q * P.nS + s, sq = s * P.nQ + q;
+  const uint64_t ab = P.qleft ? qs : sq;
+  int u = 0;
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    if (!((KEYS >> o) & 1)) continue;
+    take_cand(C, j + u, s < P.nS && ((P.mask >> o) & 1), P.gb[o] + (o < 2 ? ab : o == 2 ? qs : sq), bad[u], cnt);
+    ++u;
   }
 }
 
-template <int MODE, bool BULK>
-__device__ inline void p1_binary_keys(int keys, InstDev& I, const TileSh& P, const uint64_t* sS, int sp,
-                                      const uint64_t* sQ, P1Count& cnt) {
-  switch (keys) {
-    case 15: p1_binary<MODE, 15, BULK>(I, P, sS, sp, sQ, cnt); break;
-    case 7: p1_binary<MODE, 7, BULK>(I, P, sS, sp, sQ, cnt); break;
-    // & alone is computed with | (one variant less: a smaller kernel image
-    // measured faster on small levels)
-    default: p1_binary<MODE, 3, BULK>(I, P, sS, sp, sQ, cnt);
+// Hash keys.  Bound by instruction issue and the ALU pipe (level 8 of the large
+// instance: 5.5 M candidates of 63 words in 0.61 ms, before 1.09 ms; ALU pipe
+// 62%): per word, 11 ALU instructions for & or |, 16 for a U, and 6 multiplies
+// each.  The first xor-shift of a & b is (a & b) ^ (a >> 30 & b >> 30), so the
+// shifted words are made once per row and word, and the reversed words of U
+// too; the last xor-shift is taken once per key (splitmix_end).
+// QB staged rows at a time: two where only & and | are kept (the same four keys
+// as one row with both U), so that the stream row's loads are shared.
+template <int KEYS, int QB>
+__device__ __forceinline__ void p1_pair_hash(const TileSh& P, const uint64_t* srow, const QWord* qw, uint64_t q,
+                                             uint64_t s, Cands& C, P1Count& cnt) {
+  constexpr int N = key_count(KEYS);
+  uint64_t acc[QB][N], hi[QB][N];
+  uint32_t bad[QB][N];
+  auto each = [&](auto&& f) {
+#pragma unroll
+    for (int b = 0; b < QB; ++b)
+#pragma unroll
+      for (int j = 0; j < N; ++j) f(b, j);
+  };
+  each([&](int b, int j) {
+    acc[b][j] = hi[b][j] = 0;
+    bad[b][j] = 0;
+  });
+  const int TP = P.TP;
+  auto word = [&](int t, uint64_t sw) {
+    const uint64_t ssh = sw >> 30;
+    const uint64_t srev = (KEYS & 12) ? __brevll(sw) : 0ULL;
+#pragma unroll
+    for (int b = 0; b < QB; ++b) {
+      const QWord x = qw[b * TP + t];
+      int j = 0;
+      if (KEYS & 1) {
+        const uint64_t w = sw & x.w;
+        bad[b][j] |= lo32(w) ^ x.lab;
+        acc[b][j++] ^= splitmix_mul(w ^ (ssh & x.sh));
+      }
+      if (KEYS & 2) {
+        const uint64_t w = sw | x.w;
+        bad[b][j] |= lo32(w) ^ x.lab;
+        acc[b][j++] ^= splitmix_mul(w ^ (ssh | x.sh));
+      }
+      if (KEYS & 4) {
+        const uint64_t w = __brevll(until_rev(x.rev, srev));
+        bad[b][j] |= lo32(w) ^ x.lab;
+        acc[b][j++] ^= splitmix_mul(w ^ (w >> 30));
+      }
+      if (KEYS & 8) {
+        const uint64_t w = __brevll(until_rev(srev, x.rev));
+        bad[b][j] |= lo32(w) ^ x.lab;
+        acc[b][j++] ^= splitmix_mul(w ^ (w >> 30));
+      }
+    }
+  };
+  row_pass(srow, TP, P.half & ~1, [&](int t, uint64_t x, uint64_t y) {
+    word(t, x);
+    word(t + 1, y);
+  }, [&] { each([&](int b, int j) { hi[b][j] = acc[b][j]; }); });
+  // (h and l as in p1_unary)
+  uint64_t all[QB][N];
+  each([&](int b, int j) {
+    all[b][j] = acc[b][j];
+    acc[b][j] = 0;
+  });
+  if (P.half & 1) word(P.half - 1, ld_row1(srow + P.half - 1));
+  each([&](int b, int j) {
+    key_final<KEY_HASH>(KeyAcc{all[b][j] ^ hi[b][j] ^ acc[b][j], hi[b][j] ^ acc[b][j]}, C.h[b * N + j], C.l[b * N + j]);
+  });
+#pragma unroll
+  for (int b = 0; b < QB; ++b) take_pair<KEYS>(P, q + b, s, b * N, bad[b], C, cnt);
+}
+
+// Bit-field keys.  The key bits of a & b and a | b follow from the operands'
+// (fields and samples are taken bit by bit); those of U too when no field is
+// cut (exact: the whole candidate then costs a few dozen instructions whatever
+// the number of traces), else from U's words.  sk: the stream row's key bits.
+template <int MODE, int KEYS>
+__device__ __forceinline__ void p1_pair_bits(const TileSh& P, const uint64_t* srow, const KeyAcc& sk, const QWord* qw,
+                                             const QKey& x, uint64_t q, uint64_t s, Cands& C, P1Count& cnt) {
+  constexpr int N = key_count(KEYS);
+  uint32_t bad[N];
+  const KeyAcc kA{sk.a0 & x.k0, sk.a1 & x.k1}, kO{sk.a0 | x.k0, sk.a1 | x.k1};
+  int j = 0;
+  if (MODE == KEY_CONCAT && P.exact) {
+    if (KEYS & 1) { exact_key(P, Bits128{kA.a0, kA.a1}, C.h[j], C.l[j], bad[j]); ++j; }
+    if (KEYS & 2) { exact_key(P, Bits128{kO.a0, kO.a1}, C.h[j], C.l[j], bad[j]); ++j; }
+    if (KEYS & 12) {
+      const Bits128 nl = rev128(Bits128{~P.last[0], ~P.last[1]});
+      const Bits128 sr = rev128(Bits128{sk.a0, sk.a1}), qr{x.r0, x.r1};
+      if (KEYS & 4) {
+        exact_key(P, until_exact(Bits128{qr.a & nl.a, qr.b & nl.b}, sr), C.h[j], C.l[j], bad[j]);
+        ++j;
+      }
+      if (KEYS & 8) {
+        exact_key(P, until_exact(Bits128{sr.a & nl.a, sr.b & nl.b}, qr), C.h[j], C.l[j], bad[j]);
+        ++j;
+      }
+    }
+  } else {
+    KeyAcc k[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      key_init(k[u]);
+      bad[u] = 0;
+    }
+    auto word = [&](int t, uint64_t sw) {
+      const QWord y = qw[t];
+      int u = 0;
+      if (KEYS & 1) bad[u++] |= lo32(sw & y.w) ^ y.lab;
+      if (KEYS & 2) bad[u++] |= lo32(sw | y.w) ^ y.lab;
+      if (KEYS & 12) {
+        const uint64_t srev = __brevll(sw);
+        auto put = [&](uint64_t w) {
+          bad[u] |= lo32(w) ^ y.lab;
+          key_word<MODE>(k[u++], w, t, 0, P.off[t], P.wid[t], P.stride, P.len[t]);
+        };
+        if (KEYS & 4) put(__brevll(until_rev(y.rev, srev)));
+        if (KEYS & 8) put(__brevll(until_rev(srev, y.rev)));
+      }
+    };
+    row_pass(srow, P.TP, -1, [&](int t, uint64_t a, uint64_t b) {
+      word(t, a);
+      word(t + 1, b);
+    }, [] {});
+    if (KEYS & 1) k[j++] = kA;
+    if (KEYS & 2) k[j++] = kO;
+#pragma unroll
+    for (int u = 0; u < N; ++u) key_final<MODE>(k[u], C.h[u], C.l[u]);
   }
+  take_pair<KEYS>(P, q, s, 0, bad, C, cnt);
+}
+
+// Staged row q of a binary tile (and the next, where two are taken at a time)
+// against this thread's stream row; returns the staged rows done.  The
+// operators up to the last one kept: & and | always (& alone is computed with
+// |: a variant less, and a smaller kernel image measured faster on small
+// levels), either U, or both.
+template <int MODE>
+__device__ __forceinline__ int p1_pair(const TileSh& P, const uint64_t* srow, const KeyAcc& sk, const QWord* sQ,
+                                       const QKey* sK, int q, Cands& C, P1Count& cnt) {
+  const uint64_t s = P.s0 + threadIdx.x;
+  int done = 1;
+  auto go = [&](auto keys) {
+    constexpr int K = decltype(keys)::value;
+    const QWord* qw = sQ + q * P.TP;
+    if constexpr (MODE != KEY_HASH) {
+      p1_pair_bits<MODE, K>(P, srow, sk, qw, sK[q], P.q0 + q, s, C, cnt);
+    } else {
+      if (K == 3 && q + 1 < P.nq) {
+        p1_pair_hash<K, K == 3 ? 2 : 1>(P, srow, qw, P.q0 + q, s, C, cnt);
+        done = 2;
+      } else {
+        p1_pair_hash<K, 1>(P, srow, qw, P.q0 + q, s, C, cnt);
+      }
+    }
+  };
+  switch (P.mask & 12) {
+    case 12: go(Keys<15>{}); break;
+    case 8: go(Keys<11>{}); break;
+    case 4: go(Keys<7>{}); break;
+    default: go(Keys<3>{});
+  }
+  return done;
 }
 
 // On-the-fly level (nothing stored): the tile's candidates get the solution
 // test alone, step 0 of every trace against its label; no key, no insert.
-template <bool BULK>
-__device__ inline void p1_solutions(InstDev& I, const TileSh& P, const uint64_t* sS, int sp, const uint64_t* sQ,
-                                    P1Count& cnt) {
+__device__ inline void p1_solutions(const TileSh& P, const uint64_t* rows, const QWord* sQ, P1Count& cnt) {
   const uint64_t s = P.s0 + threadIdx.x;
-  if (s >= P.nS) return;
-  const uint64_t* srow = sS + threadIdx.x * sp;
-  if (P.kind == 0) {
+  for (int q = 0; q < P.nq; ++q) {
+    const uint64_t a = P.kind ? s : s + (uint64_t)q * kTS;
+    if (a >= P.nS) return;
+    const uint64_t* row = rows + a * P.TP;
     uint32_t bad[4] = {0, 0, 0, 0};
-    p1_words<BULK>(P, [&](int t, auto) {
-      const uint64_t w = srow[t], lm = len_mask(P.len[t]);
-      const uint32_t pb = (uint32_t)pos_bit(P, t);
-      bad[0] |= lo32(~w & lm) ^ pb;
-      bad[1] |= lo32(w >> 1) ^ pb;
-      bad[2] |= lo32(w_fin(w)) ^ pb;
-      bad[3] |= lo32(w_glob(w, lm)) ^ pb;
-    });
-    const uint64_t g[4] = {I.base_not + s, I.base_x + s, I.base_f + s, I.base_g + s};
+    uint64_t g[4];
+    if (P.kind == 0) {
+      auto word = [&](int t, uint64_t w) {
+        const TraceSh x = P.tr[t];
+        bad[0] |= lo32(~w & x.lm) ^ x.lab;
+        bad[1] |= lo32(w >> 1) ^ x.lab;
+        bad[2] |= lo32(w_fin(w)) ^ x.lab;
+        bad[3] |= lo32(w_glob(w, x.lm)) ^ x.lab;
+      };
+      row_pass(row, P.TP, -1, [&](int t, uint64_t x, uint64_t y) {
+        word(t, x);
+        word(t + 1, y);
+      }, [] {});
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (((P.mask >> j) & 1) && !(bad[j] & 1u) && g[j] < cnt.sol) cnt.sol = g[j];
-    return;
-  }
-  const int nq = (int)((P.nQ - P.q0) < (uint64_t)P.tq ? (P.nQ - P.q0) : (uint64_t)P.tq);
-  for (int q = 0; q < nq; ++q) {
-    const uint64_t* qrow = sQ + q * P.TP;
-    uint32_t bad[4] = {0, 0, 0, 0};
-    p1_words<BULK>(P, [&](int t, auto) {
-      const uint64_t qw = qrow[t], sw = srow[t];
-      const uint64_t la = P.qleft ? qw : sw, lb = P.qleft ? sw : qw;
-      const uint32_t pb = (uint32_t)pos_bit(P, t);
-      bad[0] |= lo32(la & lb) ^ pb;
-      bad[1] |= lo32(la | lb) ^ pb;
-      bad[2] |= lo32(w_until(la, lb)) ^ pb;
-      bad[3] |= lo32(w_until(lb, la)) ^ pb;
-    });
-    const uint64_t a = P.qleft ? P.q0 + q : s, b = P.qleft ? s : P.q0 + q;
-    const uint64_t ab = a * P.nj + b;
-    const uint64_t g[4] = {I.base_and[P.i] + ab, I.base_or[P.i] + ab, I.base_u[P.i] + ab, I.base_u[P.j] + b * P.ni + a};
+      for (int j = 0; j < 4; ++j) g[j] = P.gb[j] + a;
+    } else {
+      const QWord* qw = sQ + q * P.TP;
+      auto word = [&](int t, uint64_t sw) {
+        const QWord y = qw[t];
+        const uint64_t srev = __brevll(sw);
+        bad[0] |= lo32(sw & y.w) ^ y.lab;
+        bad[1] |= lo32(sw | y.w) ^ y.lab;
+        bad[2] |= lo32(__brevll(until_rev(y.rev, srev))) ^ y.lab;
+        bad[3] |= lo32(__brevll(until_rev(srev, y.rev))) ^ y.lab;
+      };
+      row_pass(row, P.TP, -1, [&](int t, uint64_t x, uint64_t y) {
+        word(t, x);
+        word(t + 1, y);
+      }, [] {});
+      const uint64_t qs = (P.q0 + q) * P.nS + s, sq = s * P.nQ + P.q0 + q, ab = P.qleft ? qs : sq;
+      g[0] = P.gb[0] + ab;
+      g[1] = P.gb[1] + ab;
+      g[2] = P.gb[2] + qs;
+      g[3] = P.gb[3] + sq;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (((P.mask >> j) & 1) && !(bad[j] & 1u) && g[j] < cnt.sol) cnt.sol = g[j];
