@@ -104,7 +104,8 @@ struct InstDev {
   uint64_t* wins;              // owners of new keys, ascending candidate index
   uint64_t tent_cap;           // capacity of wins
   // ---- search state
-  int status, level, need, pad0;
+  int status, level, need;
+  int keep_last;               // the rows of level max_size are wanted too (a BS stage follows)
   uint64_t need_amount[4];     // requested bitmap words / slots / list entries / rows
   uint64_t lstart[kMaxSize + 2];
   uint64_t lcount[kMaxSize + 2];

@@ -1043,6 +1043,7 @@ struct Engine {
     d.weighted = req_neg == 2;
     for (int c = 0; c < 8; ++c) d.weighted |= req_cost[c] > 1;
     if (atom_level(d) > d.max_size) return VFB_BAD_INPUT;
+    d.keep_last = bs_max > 0;
     d.status = ST_RUNNING;
     d.level = 1;
     return VFB_OK;

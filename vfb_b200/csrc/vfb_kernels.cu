@@ -677,12 +677,28 @@ __device__ __forceinline__ bool below_mode(const InstDev& I) {
   return I.best_cand != ~0ULL && !I.on_the_fly && !I.no_mask && !I.mask_off;
 }
 
+// Level max_size of a search (its first attempt): no later level reads its
+// rows, so none are listed or written.  Without a solution candidate after P1
+// its result is the number of its owners, which is the number of keys P1
+// published; with one, the owners below it are counted (below_mode).  A
+// failed ownership check or a buffer found too small builds the level again
+// in full.  (49 traces, size 9, nothing found: 8.7 M rows of the last level,
+// k_emit 3.2 -> 0.4 ms, the scan 0.45 -> 0.1, the solve 5.83 -> 2.9 ms.)
+__device__ __forceinline__ bool last_level(const InstDev& I) {
+  return I.level == I.max_size && I.attempt == 1 && !I.keep_last && !I.on_the_fly && !I.no_mask && !I.mask_off;
+}
+__device__ __forceinline__ bool last_unsolved(const InstDev& I) { return last_level(I) && I.best_cand == ~0ULL; }
+
+// COUNT_LAST: a last level without a solution candidate needs no scan (the
+// caller takes the count of published keys).
+template <bool COUNT_LAST>
 __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
   __shared__ unsigned long long s_w[32], s_b[32];
   const unsigned long long total = B.tscan_prefix[B.ninst];
   for (unsigned long long c = bid; c < total; c += nb) {
     const int b = find_owner(B.tscan_prefix, B.ninst, c);
     InstDev& I = B.inst[b];
+    if (COUNT_LAST && last_unsolved(I)) continue;
     const unsigned long long k = (unsigned long long)I.level;
     // first attempt at this level with every new slot listed: visit the list;
     // otherwise (a retried level) scan the whole table
@@ -778,7 +794,7 @@ __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
 
 __global__ void k_table_scan(BatchDev* Bp) {
   const BatchDev B = *Bp;
-  ph_table_scan(B, blockIdx.x, gridDim.x);
+  ph_table_scan<false>(B, blockIdx.x, gridDim.x);
 }
 
 // Graph solver: k_table_scan, then the last CTA to finish checks every
@@ -798,7 +814,7 @@ __global__ void k_table_scan_check(BatchDev* Bp) {
   if (part > gridDim.x) part = gridDim.x;
   if (part == 0) part = 1;
   if (blockIdx.x >= part) return;
-  ph_table_scan(B, blockIdx.x, (unsigned)part);
+  ph_table_scan<true>(B, blockIdx.x, (unsigned)part);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -814,7 +830,8 @@ __global__ void k_table_scan_check(BatchDev* Bp) {
     if (b < B.ninst) {
       InstDev& I = B.inst[b];
       if (*(volatile int*)&I.status == ST_RUNNING) {
-        const unsigned long long nw = *(volatile unsigned long long*)&I.n_wins;
+        const bool counted = last_unsolved(I);
+        const unsigned long long nw = counted ? I.n_new : *(volatile unsigned long long*)&I.n_wins;
         const unsigned long long fails = *(volatile unsigned long long*)&I.probe_fail;
         const int sk = *(volatile int*)&I.sol_known;
         const unsigned long long cap = I.table_mask + 1;
@@ -827,6 +844,8 @@ __global__ void k_table_scan_check(BatchDev* Bp) {
           I.need = need;
           I.planned = 0;
           I.status = ST_NEED_MEM;
+        } else if (counted) {
+          I.n_wins = nw;
         } else if (!sk) {
           const int item = nw >= kEmitItemFrom ? kEmitItem : kEmitGroup;
           I.emit_item = item;
@@ -1061,12 +1080,13 @@ __device__ void finish_one(InstDev& I) {
   const uint64_t* wlist = I.wins;
   const uint64_t n_below = I.n_below;
   const int no_list = I.no_list;
+  const bool counted = last_unsolved(I);
   const int attempt = I.attempt, sol_known = I.sol_known, max_size = I.max_size,
             counted_below = I.counted_below;
   I.built_cands = cands;
   I.built_wins = wins;
-  I.built_scanned = (attempt == 1 && !no_list && newlist <= tent) ? newlist : cap;
-  I.built_sol_known = sol_known;
+  I.built_scanned = counted ? 0 : (attempt == 1 && !no_list && newlist <= tent) ? newlist : cap;
+  I.built_sol_known = sol_known || counted;
   I.keys = keys + wins;
   if (best != ~0ULL) {
     const uint64_t g = best;
@@ -1155,7 +1175,7 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(BatchDev* Bp, cudaG
         const unsigned want = I.p1_blocks ? (unsigned)I.p1_blocks : ~0u;
         blocks = want > blocks ? want : blocks;
         if (I.p1_tail) {
-          chunks = (I.plan_words + kCompactWords - 1) / kCompactWords;
+          chunks = last_level(I) ? 0 : (I.plan_words + kCompactWords - 1) / kCompactWords;
           tchunks = I.plan_tchunks;
         }
         run = 1;
@@ -1444,7 +1464,7 @@ __global__ void __launch_bounds__(kTS) k_solve(BatchDev* Bp, unsigned int max_st
     if (!grid_sync(ctl, nb)) return;
     ph_p1(B);
     if (!grid_sync(ctl, nb)) return;
-    ph_table_scan(B, bid, nb);
+    ph_table_scan<false>(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
     ph_chunk_count(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
@@ -1507,7 +1527,7 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
       cl.sync();
       ph_p1(B);
       cl.sync();
-      ph_table_scan(B, rank, csize);
+      ph_table_scan<false>(B, rank, csize);
       cl.sync();
       ph_chunk_count(B, rank, csize);
       cl.sync();
