@@ -1336,15 +1336,54 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(BatchDev* Bp) {
 // order, solution test (insertInCache LTL_BS.cu:299-329).  Work items are
 // kEmitItem consecutive owners of one instance on large levels, kEmitGroup
 // on small ones (prefix built by k_table_scan_check, which records the
-// choice); a warp takes an item, each lane decodes one owner
-// (decode_level: compares with the plan's block bases), then the owners go
-// kEmitGroup at a time, lane per trace word, so row reads and writes stay
-// coalesced and the loads of a group's owners are in flight together.
-__global__ void __launch_bounds__(256, 3) k_emit(BatchDev* Bp) {
+// choice).  A warp takes an item: each lane decodes one owner (decode_level:
+// compares with the plan's block bases); the item's rows are one block of the
+// level cache, which the lanes write 16 bytes at a time side by side, whatever
+// the rows' pitch, kEmitUnroll pieces of their operand rows in flight.
+// Bound by HBM and instruction issue: level 9 of the large instance (24.3 M rows
+// of 64 words, about 19 GB) takes 4.5 ms; with a lane per 8-byte word, a row's
+// last words on partly idle warps, and the words' tests one by one, 7.65 ms.
+constexpr int kEmitUnroll = 4;
+constexpr int kEmitThreads = 256;
+
+// The traces as the emission needs them (per warp): length masks and labels
+// (3 for a positive trace: its own and the X test's bit).  The padding word's
+// entry repeats the last trace's.
+struct __align__(16) EmitTraces {
+  uint64_t lm[kMaxTraces];
+  uint32_t lab[kMaxTraces];
+};
+
+__device__ __forceinline__ ulonglong2 emit_words(int op, ulonglong2 l, ulonglong2 r, ulonglong2 lm, uint64_t second) {
+  switch (op) {
+    case OP_NOT: return make_ulonglong2(~l.x & lm.x, ~l.y & lm.y & second);
+    case OP_AND: return make_ulonglong2(l.x & r.x, l.y & r.y);
+    case OP_OR: return make_ulonglong2(l.x | r.x, l.y | r.y);
+    case OP_X: return make_ulonglong2(l.x >> 1, l.y >> 1);
+    case OP_F: return make_ulonglong2(w_fin(l.x), w_fin(l.y));
+    case OP_G: return make_ulonglong2(w_glob(l.x, lm.x), w_glob(l.y, lm.y));
+    default: return make_ulonglong2(w_until(l.x, r.x), w_until(l.y, r.y));
+  }
+}
+
+// emit_miss of two words (see there; a word covers its whole trace when it
+// equals the length mask).
+__device__ __forceinline__ unsigned emit_test(uint64_t w0, uint64_t w1, ulonglong2 lm, uint2 lab) {
+  const unsigned x0 = (unsigned)w0 ^ lab.x, x1 = (unsigned)w1 ^ lab.y;
+  const bool l0 = lab.x != 0, l1 = lab.y != 0;
+  const bool f = ((w0 != 0) != l0) || ((w1 != 0) != l1);
+  const bool g = ((w0 == lm.x) != l0) || ((w1 == lm.y) != l1);
+  return ((x0 | x1) & 3u) | (f ? 4u : 0u) | (g ? 8u : 0u) | ((~(x0 & x1) & 1u) << 4);
+}
+
+__global__ void __launch_bounds__(kEmitThreads, 3) k_emit(BatchDev* Bp) {
+  __shared__ EmitTraces s_tr[kEmitThreads / 32];
   step_entry();
   const BatchDev B = *Bp;
   const unsigned long long total = B.win_prefix[B.ninst];
   const int lane = threadIdx.x & 31;
+  EmitTraces& tr = s_tr[threadIdx.x >> 5];
+  int prev = -1;   // the instance tr holds
   const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   for (unsigned long long item = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < total;
        item += nw) {
@@ -1352,14 +1391,25 @@ __global__ void __launch_bounds__(256, 3) k_emit(BatchDev* Bp) {
     InstDev& I = B.inst[b];
     if (I.status != ST_RUNNING) continue;
     const int k = I.level, T = I.T, TP = I.TP;
+    if (b != prev) {
+      prev = b;
+      __syncwarp();
+      for (int t = lane; t < TP; t += 32) {
+        const int u = t < T ? t : T - 1;
+        tr.lm[t] = len_mask(I.len[u]);
+        tr.lab[t] = is_pos(I, u) ? 3u : 0u;
+      }
+      __syncwarp();
+    }
     const uint64_t per = (uint64_t)I.emit_item;
     const uint64_t o0 = (item - B.win_prefix[b]) * per;
     const uint64_t nwin = I.n_wins;
     const int cnt = (int)(nwin - o0 < per ? nwin - o0 : per);
+    const uint64_t r0 = I.lstart[k] + o0;
     // lane l decodes owner o0 + l
     int op = -1;
-    const uint64_t* pa = nullptr;
-    const uint64_t* pb = nullptr;
+    const uint64_t* pa = I.rows;
+    const uint64_t* pb = I.rows;
     uint64_t g = 0;
     if (lane < cnt) {
       g = __ldcg(I.wins + o0 + lane);
@@ -1368,51 +1418,62 @@ __global__ void __launch_bounds__(256, 3) k_emit(BatchDev* Bp) {
       if (op >= 0) {
         pa = row_ptr(I, cd.la, cd.a);
         pb = (op == OP_AND || op == OP_OR || op == OP_U) ? row_ptr(I, cd.lb, cd.b) : pa;
+        I.origin[r0 + lane] = g;
       }
     }
-    const uint64_t r0 = I.lstart[k] + o0;
-    for (int s0 = 0; s0 < cnt; s0 += kEmitGroup) {
-      int ops[kEmitGroup];
-      const uint64_t* ra[kEmitGroup];
-      const uint64_t* rb[kEmitGroup];
-      unsigned miss[kEmitGroup];   // emit_miss OR-ed over the words
+    const bool pairs = __any_sync(0xffffffffu, pb != pa);   // (an item of unary owners reads one operand)
+    // the item's rows as 16-byte units, side by side
+    const int U = TP / 2, units = cnt * U;
+    const unsigned inv = ((1u << 20) + U - 1) / U;   // f / U = f * inv >> 20 for f below 2^11
+    ulonglong2* out = reinterpret_cast<ulonglong2*>(I.rows + r0 * (uint64_t)TP);
+    unsigned miss = 0u;   // of this lane's owner: emit_miss OR-ed over its words
+    for (int f0 = 0; f0 < units; f0 += 32 * kEmitUnroll) {
+      ulonglong2 xa[kEmitUnroll], xb[kEmitUnroll];
+      int o[kEmitUnroll], un[kEmitUnroll];
 #pragma unroll
-      for (int u = 0; u < kEmitGroup; ++u) {
-        const int src = s0 + u;
-        const int o = __shfl_sync(0xffffffffu, op, src & 31);
-        ops[u] = src < cnt ? o : -1;
-        ra[u] = (const uint64_t*)__shfl_sync(0xffffffffu, (unsigned long long)pa, src & 31);
-        rb[u] = (const uint64_t*)__shfl_sync(0xffffffffu, (unsigned long long)pb, src & 31);
-        miss[u] = 0u;
-      }
-      for (int t = lane; t < TP; t += 32) {
-        const int L = t < T ? I.len[t] : 0;
-        const unsigned lab = (t < T && is_pos(I, t)) ? 1u : 0u;
-        const uint64_t lm = len_mask(L);
-        uint64_t xa[kEmitGroup], xb[kEmitGroup];
-#pragma unroll
-        for (int u = 0; u < kEmitGroup; ++u) {
-          xa[u] = (ops[u] >= 0 && t < T) ? __ldg(ra[u] + t) : 0ULL;
-          xb[u] = (ops[u] >= 0 && t < T) ? __ldg(rb[u] + t) : 0ULL;
-        }
-#pragma unroll
-        for (int u = 0; u < kEmitGroup; ++u) {
-          if (ops[u] < 0) continue;
-          const uint64_t word = t < T ? apply_w(ops[u], xa[u], xb[u], L) : 0ULL;
-          if (t < T) miss[u] |= emit_miss(word, lm, lab);
-          I.rows[(r0 + s0 + u) * (uint64_t)TP + t] = word;
+      for (int u = 0; u < kEmitUnroll; ++u) {
+        const int f = f0 + 32 * u + lane, row = (int)(((unsigned)f * inv) >> 20) & 31;
+        un[u] = f - row * U;
+        const int ro = __shfl_sync(0xffffffffu, op, row);
+        o[u] = f < units ? ro : -1;
+        const ulonglong2* a = (const ulonglong2*)__shfl_sync(0xffffffffu, (unsigned long long)pa, row);
+        xa[u] = xb[u] = make_ulonglong2(0, 0);
+        if (o[u] >= 0) xa[u] = __ldg(a + un[u]);
+        if (pairs) {
+          const ulonglong2* c = (const ulonglong2*)__shfl_sync(0xffffffffu, (unsigned long long)pb, row);
+          if (o[u] >= 0) xb[u] = __ldg(c + un[u]);
         }
       }
 #pragma unroll
-      for (int u = 0; u < kEmitGroup; ++u) {
-        if (ops[u] < 0) continue;
-        const unsigned m = __reduce_or_sync(0xffffffffu, miss[u]);
-        if (lane == s0 + u) {
-          I.origin[r0 + s0 + u] = g;
-          if (!(m & 1u)) atomicMin(&I.best_sol, (unsigned long long)g);
-          record_unary(I, k, o0 + s0 + u, ((m >> 4) & 1u) | (m & 0xEu));   // (~ X F G)
+      for (int u = 0; u < kEmitUnroll; ++u) {
+        const int f = f0 + 32 * u;
+        if (f >= units) break;   // (warp-uniform)
+        unsigned m = 0u;
+        if (o[u] >= 0) {
+          const ulonglong2 lm = reinterpret_cast<const ulonglong2*>(tr.lm)[un[u]];
+          const uint2 lab = reinterpret_cast<const uint2*>(tr.lab)[un[u]];
+          const bool pad = 2 * un[u] + 1 == T;
+          const ulonglong2 w = emit_words(o[u], xa[u], xb[u], lm, pad ? 0ULL : ~0ULL);
+          out[f + lane] = w;
+          m = emit_test(w.x, pad ? w.x : w.y, lm, lab);
+        }
+        if (U == 32) {   // a row per step
+          m = __reduce_or_sync(0xffffffffu, m);
+          if (lane == f >> 5) miss |= m;
+        } else {
+          // this lane's owner has units lane * U .. + U - 1: the lanes of this step with some of them
+          const int lo = lane * U - f, hi = lo + U;
+          const unsigned seg = (hi <= 0 || lo >= 32) ? 0u
+                               : (hi >= 32 ? ~0u : (1u << hi) - 1u) & (lo <= 0 ? ~0u : ~0u << lo);
+#pragma unroll
+          for (int j = 0; j < 5; ++j)
+            if (__ballot_sync(0xffffffffu, (m >> j) & 1u) & seg) miss |= 1u << j;
         }
       }
+    }
+    if (lane < cnt && op >= 0) {
+      if (!(miss & 1u)) atomicMin(&I.best_sol, (unsigned long long)g);
+      record_unary(I, k, o0 + lane, ((miss >> 4) & 1u) | (miss & 0xEu));   // (~ X F G)
     }
   }
 }
