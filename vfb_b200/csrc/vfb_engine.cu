@@ -482,9 +482,11 @@ struct Engine {
     }
     hB.inst = dInst;
     hB.ninst = ninst;
-    if (cudaMemcpyAsync(dB, &hB, sizeof(BatchDev), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-      return dev_fail(__LINE__);
-    c_h2d += sizeof(BatchDev);
+    if (use_coop) {   // (the other kernels take it by value)
+      if (cudaMemcpyAsync(dB, &hB, sizeof(BatchDev), cudaMemcpyHostToDevice, stream) != cudaSuccess)
+        return dev_fail(__LINE__);
+      c_h2d += sizeof(BatchDev);
+    }
     return VFB_OK;
   }
 
@@ -519,18 +521,18 @@ struct Engine {
     unsigned int mx = kMaxLoop;
     mark();
     if (pre) {
-      step_launch(false, k_advance, 1u, (unsigned)adv_threads, 0, dB, handle, built0, lp, mx);
+      step_launch(false, k_advance, 1u, (unsigned)adv_threads, 0, hB, handle, built0, lp, mx);
       mark();
     }
-    step_launch(pdl && pre, k_p1, (unsigned)p1_grid, (unsigned)kTS, (size_t)p1_smem, dB);
+    step_launch(pdl && pre, k_p1, (unsigned)p1_grid, (unsigned)kTS, (size_t)p1_smem, hB);
     mark();
-    step_launch(pdl, k_table_scan_check, (unsigned)grid, 256u, 0, dB);
+    step_launch(pdl, k_table_scan_check, (unsigned)grid, 256u, 0, hB);
     mark();
-    step_launch(pdl, k_compact, (unsigned)(sms * 8), (unsigned)kCompactThreads, 0, dB);
+    step_launch(pdl, k_compact, (unsigned)(sms * 8), (unsigned)kCompactThreads, 0, hB);
     mark();
-    step_launch(pdl, k_emit, (unsigned)emit_grid, 256u, 0, dB);
+    step_launch(pdl, k_emit, (unsigned)emit_grid, 256u, 0, hB);
     mark();
-    step_launch(pdl, k_advance, 1u, (unsigned)adv_threads, 0, dB, handle, built1, lp, mx);
+    step_launch(pdl, k_advance, 1u, (unsigned)adv_threads, 0, hB, handle, built1, lp, mx);
     mark();
   }
 
@@ -558,7 +560,7 @@ struct Engine {
       if (e == cudaSuccess) {
         e = cudaStreamBeginCaptureToGraph(stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-          k_advance<<<1, adv_threads, 0, stream>>>(dB, handle, 0, 1, kMaxLoop);
+          k_advance<<<1, adv_threads, 0, stream>>>(hB, handle, 0, 1, kMaxLoop);
           cudaGraph_t out = nullptr;
           e = cudaStreamEndCapture(stream, &out);
         }
@@ -1245,8 +1247,8 @@ struct Engine {
     }
     if (rc == VFB_OK) {
       if (profile) cudaEventRecord(ev_k[0], stream);
-      k_fill<<<grid, 256, 0, stream>>>(dB);
-      k_init<<<std::min(n, grid), 256, 0, stream>>>(dB);
+      k_fill<<<grid, 256, 0, stream>>>(hB);
+      k_init<<<std::min(n, grid), 256, 0, stream>>>(hB);
       c_launch += 2;
       if (profile) {
         cudaEventRecord(ev_k[1], stream);
@@ -1793,8 +1795,8 @@ struct Engine {
       admitted = true;
     }
     if (admitted) {
-      k_fill<<<grid, 256, 0, stream>>>(dB);
-      k_init<<<std::min(sv.cap, grid), 256, 0, stream>>>(dB);
+      k_fill<<<grid, 256, 0, stream>>>(hB);
+      k_init<<<std::min(sv.cap, grid), 256, 0, stream>>>(hB);
       c_launch += 2;
     }
     // 2. one level for every active instance

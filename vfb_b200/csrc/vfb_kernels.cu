@@ -44,11 +44,23 @@ __device__ __forceinline__ void step_entry() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// Few instances at a time: the table scan takes only the CTAs that the levels'
+// lists need (a small level's list is one CTA's: no ticket, no waiting for
+// idle ones).
+__device__ __forceinline__ bool scan_compacts(const BatchDev& B) { return B.ninst <= 4; }
+// Whether the owner bitmap of an instance's level is compacted by the last CTA
+// of the table scan (256 threads, two words each) instead of by k_compact: a
+// kernel's start, ticket and look-back (4-5 us) cost more than the level's one
+// chunk.  One CTA would take the instances of a batch in turn: few only.
+__device__ __forceinline__ bool small_compact(const BatchDev& B, const InstDev& I) {
+  return scan_compacts(B) && I.plan_words <= kCompactWords;
+}
+
 // ===================================================================== plan
 // Plan level k = I.level of a RUNNING instance: candidate-block bases, P1
 // tiling, buffer checks.  Records the plan (planned = k, plan_*) or asks the
 // host for memory (NEED_MEM, planned = 0).
-__device__ void plan_one(InstDev& I) {
+__device__ void plan_one(InstDev& I, bool few) {
   // Everything the plan reads is loaded first: the plan runs on one thread,
   // and a load issued after a store to the record waits for that store.
   const int k = I.level, weighted = I.weighted, on_the_fly = I.on_the_fly;
@@ -270,10 +282,13 @@ __device__ void plan_one(InstDev& I) {
   } else {
     I.plan_tiles = t;
     I.plan_words = words;
-    // scan chunks of kScanSlots, larger on large tables (down to 8192 chunks,
-    // chunks of at most 4 kScanSlots): fewer per-chunk reductions and atomics
-    uint64_t ss = (uint64_t)kScanSlots;
-    while (ss < 4 * (uint64_t)kScanSlots && table_cap / (2 * ss) >= 8192) ss *= 2;
+    // scan chunks of kScanSlots, larger on larger tables (8 kScanSlots while
+    // 2048 chunks remain, 32 while 8192 do): small levels spread over the SMs,
+    // large ones make fewer per-chunk reductions and atomics; the instances of
+    // a batch fill the SMs together and start at 8 kScanSlots
+    uint64_t ss = (few ? 1 : 8) * (uint64_t)kScanSlots;
+    while (ss < 8 * (uint64_t)kScanSlots && table_cap / (2 * ss) >= 2048) ss *= 2;
+    while (ss < 32 * (uint64_t)kScanSlots && table_cap / (2 * ss) >= 8192) ss *= 2;
     I.scan_slots = (uint32_t)ss;
     I.plan_tchunks = on_the_fly ? 0 : (table_cap + ss - 1) / ss;
     I.planned = k;
@@ -317,7 +332,7 @@ __device__ void ph_plan(const BatchDev& B, unsigned bid, unsigned nb) {
     InstDev& I = B.inst[b];
     unsigned long long tiles = 0, chunks = 0, tchunks = 0;
     if (I.status == ST_RUNNING) {
-      plan_one(I);
+      plan_one(I, scan_compacts(B));
       if (I.status == ST_RUNNING) {
         tiles = I.plan_tiles;
         chunks = (I.plan_words + kChunkWords - 1) / kChunkWords;
@@ -344,40 +359,40 @@ __device__ void ph_plan_prefix(const BatchDev& B) {
   for (int i = 0; i < kTickets; ++i) B.tickets[i] = 0;
 }
 
-__global__ void __launch_bounds__(1024) k_plan(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void __launch_bounds__(1024) k_plan(const __grid_constant__ BatchDev B) {
   ph_plan(B, 0, 1);
   __syncthreads();
   if (threadIdx.x == 0) ph_plan_prefix(B);
 }
 
 // ======================================================================= P1
-// The instance's part of a tile's shared parameters (thread per trace), kept
-// while a CTA's consecutive tiles are of one instance.
-__device__ void p1_instance(const InstDev& I, TileSh& P) {
-  for (int t = threadIdx.x; t < P.TP; t += blockDim.x) {
-    const int L = t < P.T ? I.len[t] : 0;
+// The instance's part of a tile's shared parameters (thread per trace, threads
+// t0 .. kTS-1), kept while a CTA's consecutive tiles are of one instance.
+__device__ void p1_instance(const InstDev& I, TileSh& P, int t0) {
+  const int T = I.T, TP = I.TP;
+  for (int t = threadIdx.x - t0; t < TP; t += kTS - t0) {
+    const int L = t < T ? I.len[t] : 0;
     P.len[t] = (uint8_t)L;
-    P.tr[t] = TraceSh{len_mask(L), t < P.T ? (uint32_t)pos_bit(P, t) : 0u, 0u};
-    P.off[t] = t < P.T ? I.off[t] : 0;
-    P.wid[t] = t < P.T ? I.width[t] : 0;
+    P.tr[t] = TraceSh{len_mask(L), t < T && is_pos(I, t) ? 1u : 0u, 0u};
+    P.off[t] = t < T ? I.off[t] : 0;
+    P.wid[t] = t < T ? I.width[t] : 0;
   }
-  if (P.exact && threadIdx.x < 32) {
+  if (exact_keys(I) && threadIdx.x < t0 + 32) {
     // masks over the key bits: a lane takes some traces, then XOR shuffles
     KeyAcc full{0, 0}, last{0, 0}, first{0, 0}, want{0, 0};
-    for (int t = threadIdx.x; t < P.T; t += 32) {
+    for (int t = threadIdx.x - t0; t < T; t += 32) {
       const int L = I.len[t], off = I.off[t];
       key_word<KEY_CONCAT>(full, len_mask(L), t, 0, off, L, 1, L);
       key_word<KEY_CONCAT>(last, 1ULL << (L - 1), t, 0, off, L, 1, L);
       key_word<KEY_CONCAT>(first, 1ULL, t, 0, off, L, 1, L);
-      key_word<KEY_CONCAT>(want, pos_bit(P, t), t, 0, off, L, 1, L);
+      key_word<KEY_CONCAT>(want, is_pos(I, t) ? 1ULL : 0ULL, t, 0, off, L, 1, L);
     }
     uint64_t v[8] = {full.a0, full.a1, last.a0, last.a1, first.a0, first.a1, want.a0, want.a1};
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] ^= __shfl_xor_sync(0xffffffffu, v[j], o);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == t0) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         P.full[j] = v[j];
@@ -387,14 +402,13 @@ __device__ void p1_instance(const InstDev& I, TileSh& P) {
       }
     }
   }
-  __syncthreads();
 }
 
 // The tile's staged rows into shared memory: their words (QWord) unless the
 // key bits alone settle the candidates, and their key bits (QKey) where keys
 // are bit fields.
-__device__ __forceinline__ void p1_stage(const InstDev& I, const TileSh& P, QWord* sQ, QKey* sK) {
-  const uint64_t* src = row_ptr(I, P.qi, P.q0);
+__device__ __forceinline__ void p1_stage(const TileSh& P, QWord* sQ, QKey* sK) {
+  const uint64_t* src = P.qrows;
   const int T = P.T, TP = P.TP;
   if (P.otf || !P.exact) {
     // (nq rows of TP words: one block, the padding words zero)
@@ -427,145 +441,152 @@ __device__ __forceinline__ void p1_stage(const InstDev& I, const TileSh& P, QWor
   }
 }
 
-__device__ void ph_p1(const BatchDev& B) {
+// A tile's parameters (warp 0; local: the tile's number within its instance's
+// level).  A chain of dependent loads is what this costs, so everything that
+// does not depend on the tile's group is read at once, one entry per lane for
+// the levels and the groups, then the group's bases.
+__device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, TileSh& P) {
+  const int lane = threadIdx.x & 31;
+  const int e1 = 2 * lane + 1, e2 = 2 * lane + 2;
+  const uint64_t done = __ldcg(&Ip->p1_done);
+  const int ngr = __ldcg(&Ip->ngroups);
+  uint64_t gp1 = e1 < kGroups ? __ldcg(&Ip->grp_prefix[e1]) : ~0ULL;
+  uint64_t gp2 = e2 < kGroups ? __ldcg(&Ip->grp_prefix[e2]) : ~0ULL;
+  const uint64_t cnt_l = __ldcg(&Ip->lcount[lane]), start_l = __ldcg(&Ip->lstart[lane]);
+  unsigned gr[2];   // groups lane, lane + 32: kind | mask << 8 | la << 16 | lb << 24
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int q = lane + 32 * u;
+    gr[u] = (unsigned)__ldcg(&Ip->grp_kind[q]) | ((unsigned)__ldcg(&Ip->grp_mask[q]) << 8) |
+            ((unsigned)__ldcg(&Ip->grp_la[q]) << 16) | ((unsigned)__ldcg(&Ip->grp_lb[q]) << 24);
+  }
+  const int k = __ldcg(&Ip->level), T = __ldcg(&Ip->T), TP = __ldcg(&Ip->TP);
+  const int stride = __ldcg(&Ip->stride1), mode = __ldcg(&Ip->key_mode), tq = __ldcg(&Ip->tq);
+  const int lensum = __ldcg(&Ip->lensum), otf = __ldcg(&Ip->on_the_fly), nolist = __ldcg(&Ip->no_list);
+  Slot* const table = (Slot*)__ldcg((const unsigned long long*)&Ip->table);
+  const uint64_t* const rows = (const uint64_t*)__ldcg((const unsigned long long*)&Ip->rows);
+  const unsigned long long tmask = __ldcg(&Ip->table_mask), keys = __ldcg(&Ip->keys);
+  const unsigned long long fails = __ldcg(&Ip->probe_fail), fresh = __ldcg(&Ip->n_new);
+  const unsigned long long best = __ldcg(&Ip->best_cand);
+  const int may_skip = !__ldcg(&Ip->no_mask) && !__ldcg(&Ip->mask_off);
+  // lane l holds group boundaries 2l+1 and 2l+2; the group is the number of
+  // boundaries at or below the tile (boundaries past the level's groups are
+  // stale: read as never reached)
+  local += done;
+  if (e1 >= ngr) gp1 = ~0ULL;
+  if (e2 >= ngr) gp2 = ~0ULL;
+  const int grp = __popc(__ballot_sync(0xffffffffu, gp1 <= local)) + __popc(__ballot_sync(0xffffffffu, gp2 <= local));
+  const int src = grp >= 1 ? (grp - 1) >> 1 : 0;
+  const uint64_t s1 = __shfl_sync(0xffffffffu, gp1, src), s2 = __shfl_sync(0xffffffffu, gp2, src);
+  const uint64_t gstart = grp == 0 ? 0 : ((grp & 1) ? s1 : s2);
+  const unsigned g0 = __shfl_sync(0xffffffffu, gr[0], grp & 31), g1 = __shfl_sync(0xffffffffu, gr[1], grp & 31);
+  const unsigned gw = grp < 32 ? g0 : g1;
+  const int kind = gw & 255, gmask = (gw >> 8) & 255, i = (gw >> 16) & 31, j = (gw >> 24) & 31;
+  const uint64_t ni = __shfl_sync(0xffffffffu, cnt_l, i), nj = __shfl_sync(0xffffffffu, cnt_l, j);
+  const uint64_t si = __shfl_sync(0xffffffffu, start_l, i), sj = __shfl_sync(0xffffffffu, start_l, j);
+  if (lane != 0) return;
+  uint64_t gb[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) gb[u] = __ldcg(&Ip->grp_base[grp][u]);
+  const uint64_t qt = kind ? __ldcg(&Ip->grp_qtiles[grp]) : 1;
+  const uint64_t within = local - gstart;
+  P.inst = b;
+  P.k = k;
+  P.T = T;
+  P.TP = TP;
+  P.half = T / 2;
+  P.stride = stride;
+  P.mode = mode;
+  P.exact = mode == KEY_CONCAT && lensum <= 126;
+  P.otf = otf;
+  P.nolist = nolist;
+  P.tab = table;
+  P.tmask = tmask;
+  // give up early once the table is known to be too small for this level
+  P.skip = !otf && ((fails != 0) || (4 * (keys + fresh) > 3 * (tmask + 1)));
+  P.kind = kind;
+  // operators whose first candidate in this tile comes after the best
+  // solution candidate found so far cannot change the result (every
+  // candidate before it is still evaluated): they are skipped
+  unsigned keep = 0xF;
+  int all = gmask;
+  if (kind == 0) {
+    const uint64_t s0 = within * tq * kTS, blocks = (ni - s0 + kTS - 1) / kTS;
+    P.nS = ni;
+    P.s0 = s0;
+    P.srows = rows + si * TP;
+    P.nq = (int)(blocks < (uint64_t)tq ? blocks : (uint64_t)tq);
+    if (may_skip && best != ~0ULL) {
+      keep = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) keep |= (gb[u] + s0 <= best ? 1u : 0u) << u;
+    }
+  } else {
+    const int qleft = (i == j) || (ni <= nj);
+    const uint64_t nS = qleft ? nj : ni, nQ = qleft ? ni : nj;
+    uint64_t sq, qr;
+    divmod64(within, qt, sq, qr);
+    const uint64_t s0 = sq * kTS, q0 = qr * tq;
+    P.qleft = qleft;
+    P.nS = nS;
+    P.nQ = nQ;
+    P.s0 = s0;
+    P.q0 = q0;
+    P.srows = rows + (qleft ? sj : si) * TP;
+    P.qrows = rows + ((qleft ? si : sj) + q0) * TP;
+    P.nq = (int)(nQ - q0 < (uint64_t)tq ? nQ - q0 : (uint64_t)tq);
+    // the U bits by the staged row's side (staged U stream, stream U staged)
+    // rather than by level
+    if (!qleft) {
+      all = (gmask & 3) | ((gmask & 4) << 1) | ((gmask & 8) >> 1);
+      const uint64_t x = gb[2];
+      gb[2] = gb[3];
+      gb[3] = x;
+    }
+    if (may_skip && best != ~0ULL) {
+      const uint64_t qs = q0 * nS + s0, sm = s0 * nQ + q0, ab = qleft ? qs : sm;
+      keep = (gb[0] + ab <= best ? 1u : 0u) | (gb[1] + ab <= best ? 2u : 0u) | (gb[2] + qs <= best ? 4u : 0u) |
+             (gb[3] + sm <= best ? 8u : 0u);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) P.gb[u] = gb[u];
+  P.mask = all & keep;
+  if (P.mask != all) *(volatile int*)&Ip->p1_masked = 1;
+}
+
+// CTA bid of nb: its first tile is tile bid, the later ones come by ticket.
+__device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ TileSh P;
   __shared__ WarpIns s_ins[kTS / 32];
-  __shared__ unsigned long long s_red[3][kTS / 32];
+  __shared__ unsigned long long s_red[3][kTS / 32], s_next;
   const unsigned long long total = B.p1_prefix[B.ninst];
   InsState S{&s_ins[threadIdx.x >> 5], nullptr, 0, 0, 0, false};
+  QKey* sK = reinterpret_cast<QKey*>(smem);
+  QWord* sQ = reinterpret_cast<QWord*>(smem) + kTQ;
   int prev = -1;   // the instance whose part of P is loaded
-  while (true) {
-    if (threadIdx.x < 32) {
-      // tile set-up by warp 0: the group boundaries are read one per lane and
-      // the remaining fields with their loads issued before any shared store,
-      // so the chain is a few memory round trips long
-      const int lane = threadIdx.x;
-      unsigned long long tile = 0;
-      if (lane == 0) tile = atomicAdd(B.tickets, 1ULL);
-      tile = __shfl_sync(0xffffffffu, tile, 0);
-      if (lane == 0) P.tile = tile;
-      if (tile < total) {
-        const int b = find_owner(B.p1_prefix, B.ninst, tile);
-        const InstDev* Ip = B.inst + b;
-        const uint64_t local = tile - B.p1_prefix[b] + __ldcg(&Ip->p1_done);
-        // lane l holds group boundaries 2l+1 and 2l+2; the group is the number
-        // of boundaries at or below the tile
-        const int e1 = 2 * lane + 1, e2 = 2 * lane + 2;
-        // (boundaries past the level's groups are stale: read as never reached)
-        const int ngr = __ldcg(&Ip->ngroups);
-        uint64_t gp1 = e1 < kGroups ? __ldcg(&Ip->grp_prefix[e1]) : ~0ULL;
-        uint64_t gp2 = e2 < kGroups ? __ldcg(&Ip->grp_prefix[e2]) : ~0ULL;
-        if (e1 >= ngr) gp1 = ~0ULL;
-        if (e2 >= ngr) gp2 = ~0ULL;
-        const int grp = __popc(__ballot_sync(0xffffffffu, gp1 <= local)) +
-                        __popc(__ballot_sync(0xffffffffu, gp2 <= local));
-        const int src = grp >= 1 ? (grp - 1) >> 1 : 0;
-        const uint64_t s1 = __shfl_sync(0xffffffffu, gp1, src), s2 = __shfl_sync(0xffffffffu, gp2, src);
-        const uint64_t gstart = grp == 0 ? 0 : ((grp & 1) ? s1 : s2);
-        if (lane == 0) {
-          const int k = __ldcg(&Ip->level), T = __ldcg(&Ip->T), TP = __ldcg(&Ip->TP);
-          const int stride = __ldcg(&Ip->stride1), mode = __ldcg(&Ip->key_mode), tq = __ldcg(&Ip->tq);
-          const uint64_t pos0 = __ldcg(&Ip->posmask[0]), pos1 = __ldcg(&Ip->posmask[1]);
-          const unsigned long long cap = __ldcg(&Ip->table_mask) + 1, keys = __ldcg(&Ip->keys);
-          const unsigned long long fails = __ldcg(&Ip->probe_fail), fresh = __ldcg(&Ip->n_new);
-          const int kind = __ldcg(&Ip->grp_kind[grp]), gmask = __ldcg(&Ip->grp_mask[grp]);
-          const int i = __ldcg(&Ip->grp_la[grp]), j = __ldcg(&Ip->grp_lb[grp]);
-          const uint64_t ni = __ldcg(&Ip->lcount[i]), nj = kind ? __ldcg(&Ip->lcount[j]) : 0;
-          const uint64_t qt = kind ? __ldcg(&Ip->grp_qtiles[grp]) : 1;
-          const unsigned long long best = __ldcg(&Ip->best_cand);
-          const int may_skip = !__ldcg(&Ip->no_mask) && !__ldcg(&Ip->mask_off);
-          uint64_t gb[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) gb[u] = __ldcg(&Ip->grp_base[grp][u]);
-          const uint64_t within = local - gstart;
-          P.inst = b;
-          P.grp = grp;
-          P.k = k;
-          P.T = T;
-          P.TP = TP;
-          P.half = T / 2;
-          P.stride = stride;
-          P.mode = mode;
-          P.exact = mode == KEY_CONCAT && __ldcg(&Ip->lensum) <= 126;
-          P.pos[0] = pos0;
-          P.pos[1] = pos1;
-          // give up early once the table is known to be too small for this level
-          P.otf = __ldcg(&Ip->on_the_fly);
-          P.nolist = __ldcg(&Ip->no_list);
-          P.skip = !P.otf && ((fails != 0) || (4 * (keys + fresh) > 3 * cap));
-          P.kind = kind;
-          // operators whose first candidate in this tile comes after the best
-          // solution candidate found so far cannot change the result (every
-          // candidate before it is still evaluated): they are skipped
-          unsigned keep = 0xF;
-          int all = gmask;
-          if (kind == 0) {
-            const uint64_t s0 = within * tq * kTS, blocks = (ni - s0 + kTS - 1) / kTS;
-            P.si = i;
-            P.nS = ni;
-            P.s0 = s0;
-            P.nq = (int)(blocks < (uint64_t)tq ? blocks : (uint64_t)tq);
-            if (may_skip && best != ~0ULL) {
-              keep = 0;
-#pragma unroll
-              for (int u = 0; u < 4; ++u) keep |= (gb[u] + s0 <= best ? 1u : 0u) << u;
-            }
-          } else {
-            const int qleft = (i == j) || (ni <= nj);
-            const uint64_t nS = qleft ? nj : ni, nQ = qleft ? ni : nj;
-            P.qleft = qleft;
-            P.si = qleft ? j : i;
-            P.qi = qleft ? i : j;
-            P.nS = nS;
-            P.nQ = nQ;
-            uint64_t sq, qr;
-            divmod64(within, qt, sq, qr);
-            const uint64_t s0 = sq * kTS, q0 = qr * tq;
-            P.s0 = s0;
-            P.q0 = q0;
-            P.nq = (int)(nQ - q0 < (uint64_t)tq ? nQ - q0 : (uint64_t)tq);
-            // the U bits by the staged row's side (staged U stream, stream U
-            // staged) rather than by level
-            if (!qleft) {
-              all = (gmask & 3) | ((gmask & 4) << 1) | ((gmask & 8) >> 1);
-              const uint64_t x = gb[2];
-              gb[2] = gb[3];
-              gb[3] = x;
-            }
-            if (may_skip && best != ~0ULL) {
-              const uint64_t qs = q0 * nS + s0, sm = s0 * nQ + q0, ab = qleft ? qs : sm;
-              keep = (gb[0] + ab <= best ? 1u : 0u) | (gb[1] + ab <= best ? 2u : 0u) |
-                     (gb[2] + qs <= best ? 4u : 0u) | (gb[3] + sm <= best ? 8u : 0u);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) P.gb[u] = gb[u];
-          P.mask = all & keep;
-          if (P.mask != all) *(volatile int*)&const_cast<InstDev*>(Ip)->p1_masked = 1;
-        }
-      }
-    }
+  for (unsigned long long tile = bid; tile < total;) {
+    const int b = find_owner(B.p1_prefix, B.ninst, tile);
+    InstDev& I = B.inst[b];
+    if (threadIdx.x < 32) p1_setup(&I, b, tile - B.p1_prefix[b], P);
+    else if (b != prev) p1_instance(I, P, 32);
+    prev = b;
     __syncthreads();
-    if (P.tile >= total) break;
-    InstDev& I = B.inst[P.inst];
-    if (P.inst != prev) {
-      prev = P.inst;
-      p1_instance(I, P);
-    }
-    QKey* sK = reinterpret_cast<QKey*>(smem);
-    QWord* sQ = reinterpret_cast<QWord*>(smem) + kTQ;
+    // (the next ticket comes back while this tile is worked on)
+    unsigned long long next = ~0ULL;
+    if (threadIdx.x == 0 && total > nb) next = nb + atomicAdd(B.tickets, 1ULL);
     P1Count cnt{0, 0, ~0ULL};
     // a tile whose every operator is skipped has nothing to do
     const bool idle = P.skip || (!P.otf && P.mask == 0);
     S.list = !P.nolist;
-    S.tab = I.table;
-    S.mask = I.table_mask;
+    S.tab = P.tab;
+    S.mask = P.tmask;
     if (!idle && P.kind == 1) {
-      p1_stage(I, P, sQ, sK);
+      p1_stage(P, sQ, sK);
       __syncthreads();
     }
-    const uint64_t* rows = row_ptr(I, P.si, 0);
+    const uint64_t* rows = P.srows;
     if (!idle && P.otf) {
       p1_solutions(P, rows, sQ, cnt);
     } else if (!idle) {
@@ -639,7 +660,9 @@ __device__ void ph_p1(const BatchDev& B) {
       s_red[1][wid] = cnt.fresh;
       s_red[2][wid] = cnt.fail;
     }
+    if (threadIdx.x == 0) s_next = next;
     __syncthreads();
+    tile = s_next;   // (written again after the next tile's first barrier)
     if (threadIdx.x == 0) {
       unsigned long long m = ~0ULL, f = 0, x = 0;
       for (int w = 0; w < kTS / 32; ++w) {
@@ -652,17 +675,16 @@ __device__ void ph_p1(const BatchDev& B) {
       if (P.skip) x += 1;
       if (x) atomicAdd(&I.probe_fail, x);
     }
-    __syncthreads();
+    // (thread 0 is of the warp that sets the next tile up; no other warp reads
+    // P or s_red before that tile's first barrier)
   }
 }
 
-__global__ void __launch_bounds__(kTS, 4) k_p1(BatchDev* Bp) {
+__global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev B) {
   step_entry();
-  const BatchDev B = *Bp;
-  if (blockIdx.x >= B.p1_prefix[B.ninst]) return;   // more CTAs than tiles: no ticket needed
-  const unsigned long long cap = B.tickets[kTicketP1Blocks];
-  if (cap && blockIdx.x >= cap) return;               // the tuned CTA count of this step
-  ph_p1(B);
+  const unsigned long long cap = B.tickets[kTicketP1Blocks];   // the tuned CTA count of this step
+  const unsigned nb = cap && cap < gridDim.x ? (unsigned)cap : gridDim.x;
+  if (blockIdx.x < nb) ph_p1(B, blockIdx.x, nb);
 }
 
 // ============================================================== table scan
@@ -689,72 +711,96 @@ __device__ __forceinline__ bool last_level(const InstDev& I) {
 }
 __device__ __forceinline__ bool last_unsolved(const InstDev& I) { return last_level(I) && I.best_cand == ~0ULL; }
 
-// COUNT_LAST: a last level without a solution candidate needs no scan (the
-// caller takes the count of published keys).
-template <bool COUNT_LAST>
-__device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
+// What the scan of an instance's level visits: on the first attempt, when
+// every new slot is listed, the list; otherwise the whole table.
+struct ScanJob {
+  uint64_t entries, chunk;
+  bool listed;
+};
+__device__ __forceinline__ ScanJob scan_job(const InstDev& I) {
+  ScanJob J;
+  J.listed = I.attempt == 1 && !I.no_list && I.n_newlist <= I.tent_cap;
+  J.entries = J.listed ? I.n_newlist : I.table_mask + 1;
+  J.chunk = I.scan_slots;
+  return J;
+}
+
+// Entries s0 .. s1-1 of the scan, by one CTA.
+__device__ void scan_chunk(InstDev& I, bool listed, uint64_t s0, uint64_t s1) {
   __shared__ unsigned long long s_w[32], s_b[32];
+  const unsigned long long k = (unsigned long long)I.level;
+  // a level with a solution candidate (where it may skip operators) counts
+  // the owners below the candidate instead of marking owner bits: if the
+  // candidate owns its key (nearly always, and always with exact keys)
+  // that count is all the level needs; if not, the level is built again in
+  // full (the ownership check below)
+  const unsigned long long bc = I.best_cand;
+  const bool below = below_mode(I);
+  unsigned long long cnt = 0, nbelow = 0;
+  // kScanBatch entries per thread at a time: their list reads, then their
+  // payload reads, are in flight together
+  for (uint64_t e0 = s0 + threadIdx.x; e0 < s1; e0 += (uint64_t)kScanBatch * blockDim.x) {
+    uint64_t sl[kScanBatch];
+    unsigned long long pay[kScanBatch];
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u) {
+      const uint64_t e = e0 + (uint64_t)u * blockDim.x;
+      sl[u] = e < s1 ? (listed ? __ldcg(I.wins + e) : e) : ~0ULL;
+    }
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u) pay[u] = sl[u] != ~0ULL ? __ldcg(&I.table[sl[u]].pay) : ~0ULL;
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u) {
+      if ((pay[u] >> kPayShift) == k) {
+        const uint64_t g = pay[u] & kIdxMask;
+        if (below) nbelow += g < bc ? 1 : 0;
+        else atomicOr(I.bitmap + (g >> 5), 1u << (g & 31));
+        ++cnt;
+      }
+    }
+  }
+  cnt = warp_sum(cnt);
+  nbelow = warp_sum(nbelow);
+  if ((threadIdx.x & 31) == 0) {
+    s_w[threadIdx.x >> 5] = cnt;
+    s_b[threadIdx.x >> 5] = nbelow;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t = 0, tb = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      t += s_w[w];
+      tb += s_b[w];
+    }
+    if (t) atomicAdd(&I.n_wins, t);
+    if (tb) atomicAdd(&I.n_below, tb);
+  }
+  __syncthreads();
+}
+
+// Every instance's scan, chunks of all instances side by side.  COUNT_LAST: a
+// last level without a solution candidate needs no scan (the caller takes the
+// count of published keys).
+template <bool COUNT_LAST>
+__device__ void ph_scan_tables(const BatchDev& B, unsigned bid, unsigned nb) {
   const unsigned long long total = B.tscan_prefix[B.ninst];
   for (unsigned long long c = bid; c < total; c += nb) {
     const int b = find_owner(B.tscan_prefix, B.ninst, c);
     InstDev& I = B.inst[b];
     if (COUNT_LAST && last_unsolved(I)) continue;
-    const unsigned long long k = (unsigned long long)I.level;
-    // first attempt at this level with every new slot listed: visit the list;
-    // otherwise (a retried level) scan the whole table
-    const bool listed = I.attempt == 1 && !I.no_list && I.n_newlist <= I.tent_cap;
-    const uint64_t ss = I.scan_slots;
-    const uint64_t s0 = (c - B.tscan_prefix[b]) * ss;
-    const uint64_t cap = listed ? I.n_newlist : I.table_mask + 1;
-    const uint64_t s1 = (s0 + ss < cap) ? s0 + ss : cap;
-    // a level with a solution candidate (where it may skip operators) counts
-    // the owners below the candidate instead of marking owner bits: if the
-    // candidate owns its key (nearly always, and always with exact keys)
-    // that count is all the level needs; if not, the level is built again in
-    // full (the ownership check below)
-    const unsigned long long bc = I.best_cand;
-    const bool below = below_mode(I);
-    unsigned long long cnt = 0, nbelow = 0;
-    // kScanBatch entries per thread at a time: their list reads, then their
-    // payload reads, are in flight together
-    for (uint64_t e0 = s0 + threadIdx.x; e0 < s1; e0 += (uint64_t)kScanBatch * blockDim.x) {
-      uint64_t sl[kScanBatch];
-      unsigned long long pay[kScanBatch];
-#pragma unroll
-      for (int u = 0; u < kScanBatch; ++u) {
-        const uint64_t e = e0 + (uint64_t)u * blockDim.x;
-        sl[u] = e < s1 ? (listed ? __ldcg(I.wins + e) : e) : ~0ULL;
-      }
-#pragma unroll
-      for (int u = 0; u < kScanBatch; ++u) pay[u] = sl[u] != ~0ULL ? __ldcg(&I.table[sl[u]].pay) : ~0ULL;
-#pragma unroll
-      for (int u = 0; u < kScanBatch; ++u) {
-        if ((pay[u] >> kPayShift) == k) {
-          const uint64_t g = pay[u] & kIdxMask;
-          if (below) nbelow += g < bc ? 1 : 0;
-          else atomicOr(I.bitmap + (g >> 5), 1u << (g & 31));
-          ++cnt;
-        }
-      }
+    ScanJob J = scan_job(I);
+    if (J.listed) {
+      // the list spread over the instance's chunks, at least a thread's entry each
+      const uint64_t nc = B.tscan_prefix[b + 1] - B.tscan_prefix[b], each = (J.entries + nc - 1) / nc;
+      if (each < J.chunk) J.chunk = (each + blockDim.x - 1) / blockDim.x * blockDim.x;
     }
-    cnt = warp_sum(cnt);
-    nbelow = warp_sum(nbelow);
-    if ((threadIdx.x & 31) == 0) {
-      s_w[threadIdx.x >> 5] = cnt;
-      s_b[threadIdx.x >> 5] = nbelow;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long t = 0, tb = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        t += s_w[w];
-        tb += s_b[w];
-      }
-      if (t) atomicAdd(&I.n_wins, t);
-      if (tb) atomicAdd(&I.n_below, tb);
-    }
-    __syncthreads();
+    const uint64_t s0 = (c - B.tscan_prefix[b]) * J.chunk;
+    if (s0 >= J.entries) continue;   // (uniform over the CTA)
+    scan_chunk(I, J.listed, s0, s0 + J.chunk < J.entries ? s0 + J.chunk : J.entries);
   }
+}
+
+__device__ void ph_settle_solutions(const BatchDev& B, unsigned bid, unsigned nb) {
   // solution candidate ownership (warp per instance)
   const int lane = threadIdx.x & 31;
   const unsigned long long gw = ((unsigned long long)bid * blockDim.x + threadIdx.x) >> 5;
@@ -792,67 +838,147 @@ __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_table_scan(BatchDev* Bp) {
-  const BatchDev B = *Bp;
-  ph_table_scan<false>(B, blockIdx.x, gridDim.x);
+__device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
+  ph_scan_tables<false>(B, bid, nb);
+  ph_settle_solutions(B, bid, nb);
 }
 
-// Graph solver: k_table_scan, then the last CTA to finish checks every
+__global__ void k_table_scan(const __grid_constant__ BatchDev B) {
+  ph_table_scan(B, blockIdx.x, gridDim.x);
+}
+
+// A level's buffers against its nw owners: a shortfall asks the host for
+// memory before anything of the level is written (returns false).
+__device__ bool check_buffers(InstDev& I, unsigned long long nw, int sk) {
+  const unsigned long long fails = *(volatile unsigned long long*)&I.probe_fail;
+  const unsigned long long cap = I.table_mask + 1;
+  const int k = I.level;
+  int need = 0;
+  if (fails != 0 || 4 * (I.keys + nw) > 3 * cap) { need |= NEED_TABLE; I.need_amount[1] = 4 * (I.keys + nw) + 4096; }
+  if (nw > I.tent_cap) { need |= NEED_LIST; I.need_amount[2] = nw; }
+  if (!sk && I.lstart[k] + nw > I.row_cap) { need |= NEED_ROWS; I.need_amount[3] = I.lstart[k] + nw; }
+  if (!need) return true;
+  I.need = need;
+  I.planned = 0;
+  I.status = ST_NEED_MEM;
+  return false;
+}
+
+// An instance's part of the check: its row-emission items.
+__device__ unsigned long long check_level(InstDev& I) {
+  if (*(volatile int*)&I.status != ST_RUNNING) return 0;
+  const bool counted = last_unsolved(I);
+  const unsigned long long nw = counted ? I.n_new : *(volatile unsigned long long*)&I.n_wins;
+  const int sk = *(volatile int*)&I.sol_known;
+  if (!check_buffers(I, nw, sk)) return 0;
+  if (counted) I.n_wins = nw;
+  if (counted || sk) return 0;
+  int item = kEmitGroup;
+  while (item < kEmitItem && nw > (unsigned long long)item * kEmitItemsFrom) item *= 2;
+  I.emit_item = item;
+  return (nw + item - 1) / item;
+}
+
+// The check of few instances (see scan_compacts), by one CTA: their items'
+// prefix, and their small levels' owner bitmaps into the owner lists.  The
+// bitmap's words are read while thread 0 checks the buffers.
+__device__ void check_few(const BatchDev& B, unsigned long long* s_w) {
+  __shared__ int s_go;
+  unsigned long long items = 0;
+  for (int b = 0; b < B.ninst; ++b) {
+    InstDev& I = B.inst[b];
+    const int st = *(volatile int*)&I.status;
+    const bool small = (st == ST_RUNNING || st == ST_NEED_MEM) && I.p1_tail && small_compact(B, I);
+    uint32_t v[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint64_t w = 2 * threadIdx.x + j;
+      v[j] = small && w < I.plan_words ? __ldcg(I.bitmap + w) : 0u;
+      if (v[j]) I.bitmap[w] = 0u;
+    }
+    if (threadIdx.x == 0) {
+      items += check_level(I);
+      B.win_prefix[b + 1] = items;
+      s_go = small && *(volatile int*)&I.status == ST_RUNNING;
+    }
+    unsigned long long tot, pos = block_excl_scan(__popc(v[0]) + __popc(v[1]), s_w, tot);   // (barriers)
+    if (s_go) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        for (uint32_t bits = v[j]; bits; bits &= bits - 1)
+          I.wins[pos++] = (2 * threadIdx.x + j) * 32 + __ffs(bits) - 1;
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) B.win_prefix[0] = 0;
+}
+
+// Graph solver: the table scan, then the last CTA to finish checks every
 // instance's buffers against its owner count (a shortfall asks the host for
 // memory before anything of the level is written) and builds the prefix of
-// row-emission items (kEmitItem owners each) over the instances.
-__global__ void k_table_scan_check(BatchDev* Bp) {
+// row-emission items over the instances.  CTAs beyond the level's scan chunks
+// (but at least one, and enough warps for the per-instance settle) leave at
+// once and take no ticket.
+__global__ void __launch_bounds__(kScanThreadsCheck) k_table_scan_check(const __grid_constant__ BatchDev B) {
   __shared__ int s_last;
   __shared__ unsigned long long s_w[32], s_carry;
   step_entry();
-  const BatchDev B = *Bp;
-  // CTAs beyond the level's scan chunks (but at least one, and enough warps
-  // for the per-instance settle) leave at once and take no ticket
-  const unsigned long long chunks = B.tscan_prefix[B.ninst];
-  const unsigned long long want = (unsigned long long)(B.ninst + (blockDim.x >> 5) - 1) / (blockDim.x >> 5);
-  unsigned long long part = chunks > want ? chunks : want;
+  const bool few = scan_compacts(B);
+  unsigned long long part;
+  if (few) {
+    // chunks as the levels need them: a list of up to kListChunk slots takes one CTA
+    part = 1;
+    for (int b = 0; b < B.ninst; ++b) {
+      const InstDev& I = B.inst[b];
+      if (I.status != ST_RUNNING || !I.p1_tail || I.on_the_fly || last_unsolved(I)) continue;
+      const ScanJob J = scan_job(I);
+      const uint64_t ch = J.listed ? kListChunk : J.chunk, nc = (J.entries + ch - 1) / ch;
+      part = nc > part ? nc : part;
+    }
+  } else {
+    const unsigned long long chunks = B.tscan_prefix[B.ninst];
+    const unsigned long long want = (unsigned long long)(B.ninst + (blockDim.x >> 5) - 1) / (blockDim.x >> 5);
+    part = chunks > want ? chunks : want;
+    if (part == 0) part = 1;
+  }
   if (part > gridDim.x) part = gridDim.x;
-  if (part == 0) part = 1;
   if (blockIdx.x >= part) return;
-  ph_table_scan<true>(B, blockIdx.x, (unsigned)part);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(B.tickets + 1, 1ULL) == part - 1;
-    s_carry = 0;
+  if (few) {
+    for (int b = 0; b < B.ninst; ++b) {
+      InstDev& I = B.inst[b];
+      if (I.status != ST_RUNNING || !I.p1_tail || I.on_the_fly || last_unsolved(I)) continue;
+      const ScanJob J = scan_job(I);
+      const uint64_t ch = J.listed ? kListChunk : J.chunk;
+      for (uint64_t s0 = blockIdx.x * ch; s0 < J.entries; s0 += part * ch)
+        scan_chunk(I, J.listed, s0, s0 + ch < J.entries ? s0 + ch : J.entries);
+    }
+  } else {
+    ph_scan_tables<true>(B, blockIdx.x, (unsigned)part);
+    ph_settle_solutions(B, blockIdx.x, (unsigned)part);
   }
   __syncthreads();
-  if (!s_last) return;
-  __threadfence();
+  if (part > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(B.tickets + 1, 1ULL) == part - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+  }
+  if (few) {
+    // (settled here, not before: every CTA derives part from the records, which
+    // a failed ownership check changes)
+    ph_settle_solutions(B, 0, 1);
+    __syncthreads();
+    check_few(B, s_w);
+    return;
+  }
+  if (threadIdx.x == 0) s_carry = 0;
+  __syncthreads();
   for (int base = 0; base < B.ninst; base += blockDim.x) {
     const int b = base + threadIdx.x;
-    unsigned long long groups = 0;
-    if (b < B.ninst) {
-      InstDev& I = B.inst[b];
-      if (*(volatile int*)&I.status == ST_RUNNING) {
-        const bool counted = last_unsolved(I);
-        const unsigned long long nw = counted ? I.n_new : *(volatile unsigned long long*)&I.n_wins;
-        const unsigned long long fails = *(volatile unsigned long long*)&I.probe_fail;
-        const int sk = *(volatile int*)&I.sol_known;
-        const unsigned long long cap = I.table_mask + 1;
-        const int k = I.level;
-        int need = 0;
-        if (fails != 0 || 4 * (I.keys + nw) > 3 * cap) { need |= NEED_TABLE; I.need_amount[1] = 4 * (I.keys + nw) + 4096; }
-        if (nw > I.tent_cap) { need |= NEED_LIST; I.need_amount[2] = nw; }
-        if (!sk && I.lstart[k] + nw > I.row_cap) { need |= NEED_ROWS; I.need_amount[3] = I.lstart[k] + nw; }
-        if (need) {
-          I.need = need;
-          I.planned = 0;
-          I.status = ST_NEED_MEM;
-        } else if (counted) {
-          I.n_wins = nw;
-        } else if (!sk) {
-          const int item = nw >= kEmitItemFrom ? kEmitItem : kEmitGroup;
-          I.emit_item = item;
-          groups = (nw + item - 1) / item;
-        }
-      }
-    }
+    const unsigned long long groups = b < B.ninst ? check_level(B.inst[b]) : 0;
     unsigned long long tot;
     const unsigned long long ex = block_excl_scan(groups, s_w, tot);
     if (b < B.ninst) B.win_prefix[b + 1] = s_carry + ex + groups;
@@ -889,8 +1015,7 @@ __device__ void ph_chunk_count(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_chunk_count(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void k_chunk_count(const __grid_constant__ BatchDev B) {
   ph_chunk_count(B, blockIdx.x, gridDim.x);
 }
 
@@ -951,8 +1076,7 @@ __device__ void ph_chunk_scan(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_chunk_scan(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void k_chunk_scan(const __grid_constant__ BatchDev B) {
   ph_chunk_scan(B, blockIdx.x, gridDim.x);
 }
 
@@ -998,8 +1122,7 @@ __device__ void ph_chunk_emit(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const __grid_constant__ BatchDev B) {
   ph_chunk_emit(B, blockIdx.x, gridDim.x);
 }
 
@@ -1041,8 +1164,7 @@ __device__ void ph_emit_rows(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_emit_rows(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void k_emit_rows(const __grid_constant__ BatchDev B) {
   ph_emit_rows(B, blockIdx.x, gridDim.x);
 }
 
@@ -1123,8 +1245,7 @@ __device__ void ph_finish(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_finish(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void k_finish(const __grid_constant__ BatchDev B) {
   ph_finish(B, blockIdx.x, gridDim.x);
 }
 
@@ -1134,14 +1255,13 @@ __global__ void k_finish(BatchDev* Bp) {
 // instance not yet planned for its current level is planned.  The batch's
 // tile and chunk prefixes are rebuilt from the recorded plans, the
 // look-back states of k_compact cleared and the work tickets reset.
-__global__ void __launch_bounds__(kAdvanceThreads) k_advance(BatchDev* Bp, cudaGraphConditionalHandle handle, int built,
+__global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_constant__ BatchDev B, cudaGraphConditionalHandle handle, int built,
                                                   int loop, unsigned int max_iter) {
   __shared__ int s_run, s_need;
   __shared__ unsigned s_blocks;
   __shared__ unsigned long long s_w3[32][3];
   __shared__ unsigned long long s_carry[3];
   step_entry();
-  const BatchDev B = *Bp;
   if (threadIdx.x == 0) {
     s_run = 0;
     s_need = 0;
@@ -1160,7 +1280,7 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(BatchDev* Bp, cudaG
         if (I.p1_tail) finish_one(I);
         else I.p1_done += I.p1_step;   // a slice of the level's tiles ran
       }
-      if (I.status == ST_RUNNING && I.planned != I.level) plan_one(I);
+      if (I.status == ST_RUNNING && I.planned != I.level) plan_one(I, scan_compacts(B));
       if (I.status == ST_RUNNING) {
         // this step's slice of P1 tiles: all that remain, or the quota's worth
         const unsigned long long left = I.plan_tiles - I.p1_done;
@@ -1175,7 +1295,7 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(BatchDev* Bp, cudaG
         const unsigned want = I.p1_blocks ? (unsigned)I.p1_blocks : ~0u;
         blocks = want > blocks ? want : blocks;
         if (I.p1_tail) {
-          chunks = last_level(I) ? 0 : (I.plan_words + kCompactWords - 1) / kCompactWords;
+          chunks = last_level(I) || small_compact(B, I) ? 0 : (I.plan_words + kCompactWords - 1) / kCompactWords;
           tchunks = I.plan_tchunks;
         }
         run = 1;
@@ -1235,12 +1355,11 @@ constexpr unsigned long long kFlagCount = 1ULL << 62, kFlagPrefix = 2ULL << 62;
 constexpr unsigned long long kStateMask = (1ULL << 62) - 1;
 constexpr long long kLookbackCycles = 2000000000LL;   // ~1 s: a predecessor that never publishes
 
-__global__ void __launch_bounds__(kCompactThreads) k_compact(BatchDev* Bp) {
+__global__ void __launch_bounds__(kCompactThreads) k_compact(const __grid_constant__ BatchDev B) {
   __shared__ unsigned long long s_w[32];
   __shared__ unsigned long long s_c, s_prefix;
   __shared__ int s_ok;
   step_entry();
-  const BatchDev B = *Bp;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned long long total = B.chunk_prefix[B.ninst];
   if (blockIdx.x >= total) return;   // no chunk for this CTA (small levels)
@@ -1376,10 +1495,9 @@ __device__ __forceinline__ unsigned emit_test(uint64_t w0, uint64_t w1, ulonglon
   return ((x0 | x1) & 3u) | (f ? 4u : 0u) | (g ? 8u : 0u) | ((~(x0 & x1) & 1u) << 4);
 }
 
-__global__ void __launch_bounds__(kEmitThreads, 3) k_emit(BatchDev* Bp) {
+__global__ void __launch_bounds__(kEmitThreads, 3) k_emit(const __grid_constant__ BatchDev B) {
   __shared__ EmitTraces s_tr[kEmitThreads / 32];
   step_entry();
-  const BatchDev B = *Bp;
   const unsigned long long total = B.win_prefix[B.ninst];
   const int lane = threadIdx.x & 31;
   EmitTraces& tr = s_tr[threadIdx.x >> 5];
@@ -1523,9 +1641,9 @@ __global__ void __launch_bounds__(kTS) k_solve(BatchDev* Bp, unsigned int max_st
     if (!grid_sync(ctl, nb)) return;
     if (bid == 0 && threadIdx.x == 0) ph_plan_prefix(B);
     if (!grid_sync(ctl, nb)) return;
-    ph_p1(B);
+    ph_p1(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
-    ph_table_scan<false>(B, bid, nb);
+    ph_table_scan(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
     ph_chunk_count(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
@@ -1586,9 +1704,9 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
       cl.sync();
       if (rank == 0 && threadIdx.x == 0) ph_plan_prefix(B);
       cl.sync();
-      ph_p1(B);
+      ph_p1(B, rank, csize);
       cl.sync();
-      ph_table_scan<false>(B, rank, csize);
+      ph_table_scan(B, rank, csize);
       cl.sync();
       ph_chunk_count(B, rank, csize);
       cl.sync();
@@ -1608,8 +1726,7 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
 // First buffers of new instances (fill set by the host): empty table (every
 // word ~0) and clear owner bitmap, every thread of the grid on one instance
 // after the other.
-__global__ void k_fill(BatchDev* Bp) {
-  const BatchDev B = *Bp;
+__global__ void k_fill(const __grid_constant__ BatchDev B) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
   for (int b = 0; b < B.ninst; ++b) {
@@ -1626,10 +1743,9 @@ __global__ void k_fill(BatchDev* Bp) {
 // Level 1: every proposition is a row (duplicates included); its key enters
 // the set; propositions are tested as size-1 solutions in order
 // (LTL_BS.cu:1127-1163, hashSetsInitialisation 136-160).
-__global__ void k_init(BatchDev* Bp) {
+__global__ void k_init(const __grid_constant__ BatchDev B) {
   __shared__ unsigned long long s_first;
   __shared__ unsigned long long s_new;
-  const BatchDev B = *Bp;
   for (int b = blockIdx.x; b < B.ninst; b += gridDim.x) {
     InstDev& I = B.inst[b];
     if (I.status != ST_RUNNING || I.level != 1) continue;

@@ -7,8 +7,10 @@ namespace vfb {
 constexpr int kChunkWords = 4096;     // bitmap words per compaction chunk (131072 bits)
 constexpr int kChunkThreads = 256;    // threads per compaction CTA
 constexpr int kScanThreads = 1024;
-constexpr int kScanSlots = 8192;      // hash-set slots per table-scan chunk (at least; more on
-                                      // tables of over 2^26 slots, see scan_slots)
+constexpr int kScanSlots = 1024;      // hash-set slots per table-scan chunk (at least; more on
+                                      // larger tables, see scan_slots)
+constexpr int kScanThreadsCheck = 256; // threads per k_table_scan_check CTA
+constexpr uint64_t kListChunk = 1024; // listed slots per table-scan chunk when few instances run
 constexpr int kScanBatch = 8;         // table-scan entries a thread reads at a time
 constexpr int kCompactWords = 512;    // owner-bitmap words per k_compact chunk (16384 candidates)
 constexpr int kCompactThreads = 256;  // threads per k_compact CTA (two bitmap words each)
@@ -18,10 +20,10 @@ constexpr int kAdvanceThreads = 256;
 constexpr int kTickets = 8;            // words of BatchDev::tickets
 constexpr int kTicketP1Blocks = 4;     // tickets[4]: CTAs the step's k_p1 runs (0: all), set by k_advance
 constexpr int kEmitGroup = 4;         // owners per warp step of k_emit (their loads in flight together)
-constexpr int kEmitItem = 32;         // owners per k_emit work item on large levels (one warp; a lane
-                                      // decodes each); small levels take kEmitGroup per item so that
-                                      // their few owners still spread over many warps
-constexpr unsigned long long kEmitItemFrom = 1ULL << 18;   // owners from which items are kEmitItem
+constexpr int kEmitItem = 32;         // owners per k_emit work item at most (one warp; a lane
+                                      // decodes each); small levels take as few as kEmitGroup so
+                                      // that their owners still spread over many warps
+constexpr unsigned long long kEmitItemsFrom = 4736;   // items (32 warps an SM) from which they are doubled
 
 // Staged rows of a P1 tile at most, and the dynamic shared memory of k_p1 for
 // rows of up to TP words: the staged rows' key bits and words (32 bytes each,
@@ -31,8 +33,9 @@ __host__ __device__ constexpr int p1_rows_max(int TP) { return TP > 64 ? 2 : TP 
 __host__ __device__ constexpr int p1_smem_bytes(int TP) { return 32 * (kTQ + (TP > 16 ? 264 : kTQ * TP)); }
 static_assert(p1_rows_max(128) * 128 <= 264 && p1_rows_max(64) * 64 <= 264 && p1_rows_max(32) * 32 <= 264, "");
 
-// Global batch descriptor, resident in device memory so that buffer growth
-// never invalidates a captured launch sequence.
+// Global batch descriptor, passed by value (a load less at the head of every
+// kernel); the instance records it points to stay in place when buffers grow,
+// and a captured launch sequence is built again when the workspace moves.
 struct BatchDev {
   InstDev* inst;
   int ninst;
@@ -64,22 +67,22 @@ struct BatchDev {
 // k_plan + the loop control.  With loop != 0 it sets the graph's while
 // condition: some instance RUNNING, none waiting for memory, fewer than
 // max_iter steps.
-__global__ void k_advance(BatchDev* B, cudaGraphConditionalHandle handle, int built, int loop,
+__global__ void k_advance(const __grid_constant__ BatchDev B, cudaGraphConditionalHandle handle, int built, int loop,
                           unsigned int max_iter);
-__global__ void k_table_scan_check(BatchDev* B);
-__global__ void k_compact(BatchDev* B);
-__global__ void k_emit(BatchDev* B);
+__global__ void k_table_scan_check(const __grid_constant__ BatchDev B);
+__global__ void k_compact(const __grid_constant__ BatchDev B);
+__global__ void k_emit(const __grid_constant__ BatchDev B);
 
 // Level-step kernels of the persistent, cluster and allocation-free solvers,
 // launched in this order for every level.
-__global__ void k_plan(BatchDev* B);
-__global__ void k_p1(BatchDev* B);
-__global__ void k_table_scan(BatchDev* B);
-__global__ void k_chunk_count(BatchDev* B);
-__global__ void k_chunk_scan(BatchDev* B);
-__global__ void k_chunk_emit(BatchDev* B);
-__global__ void k_emit_rows(BatchDev* B);
-__global__ void k_finish(BatchDev* B);
+__global__ void k_plan(const __grid_constant__ BatchDev B);
+__global__ void k_p1(const __grid_constant__ BatchDev B);
+__global__ void k_table_scan(const __grid_constant__ BatchDev B);
+__global__ void k_chunk_count(const __grid_constant__ BatchDev B);
+__global__ void k_chunk_scan(const __grid_constant__ BatchDev B);
+__global__ void k_chunk_emit(const __grid_constant__ BatchDev B);
+__global__ void k_emit_rows(const __grid_constant__ BatchDev B);
+__global__ void k_finish(const __grid_constant__ BatchDev B);
 
 // Persistent solver: the whole level loop in one cooperative launch (all CTAs
 // co-resident), the phases above separated by a bounded grid barrier.  Runs at
@@ -162,8 +165,8 @@ __global__ void k_bs_bounds(BsDev D, unsigned long long nent, const unsigned lon
 __global__ void k_bs_leaves(const InstDev* I, const unsigned long long* rows, int n, int16_t* rpn, int* len);
 
 // Set-up and maintenance kernels.
-__global__ void k_fill(BatchDev* B);
-__global__ void k_init(BatchDev* B);
+__global__ void k_fill(const __grid_constant__ BatchDev B);
+__global__ void k_init(const __grid_constant__ BatchDev B);
 __global__ void k_rehash(const Slot* old_tab, unsigned long long old_cap, Slot* new_tab,
                          unsigned long long new_mask, unsigned long long* fail);
 

@@ -219,7 +219,7 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
 
   // carve the static array
   Carver cv{base};
-  BatchDev* dB = cv.take<BatchDev>(1);
+  cv.take<BatchDev>(1);   // (unused: the arrays after it stay where they were, and so the rows that fit)
   InstDev* dI = cv.take<InstDev>(1);
   BatchDev hB{};
   hB.inst = dI;
@@ -266,9 +266,8 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
     ++launches;
     ok = cudaGetLastError() == cudaSuccess;
   }
-  ok = ok && cudaMemcpy(dI, &d, sizeof(InstDev), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(dB, &hB, sizeof(BatchDev), cudaMemcpyHostToDevice) == cudaSuccess;
-  h2d += sizeof(InstDev) + sizeof(BatchDev);
+  ok = ok && cudaMemcpy(dI, &d, sizeof(InstDev), cudaMemcpyHostToDevice) == cudaSuccess;
+  h2d += sizeof(InstDev);
   if (!ok) return out->status = VFB_DEVICE_ERROR;
 
   int sms = 0;
@@ -279,7 +278,7 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, p1_smem);
   const int p1_grid = sms * (occ > 0 ? occ : 1);
 
-  k_init<<<1, 256, 0, st>>>(dB);
+  k_init<<<1, 256, 0, st>>>(hB);
   ++launches;
   int2 status{ST_RUNNING, 0};
   for (int step = 0; step <= kMaxSize + 1; ++step) {
@@ -287,14 +286,14 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
       return out->status = VFB_DEVICE_ERROR;
     d2h += sizeof(int2);
     if (status.x != ST_RUNNING) break;
-    k_plan<<<1, 1024, 0, st>>>(dB);
-    k_p1<<<p1_grid, kTS, p1_smem, st>>>(dB);
-    k_table_scan<<<g, 256, 0, st>>>(dB);
-    k_chunk_count<<<gc, 256, 0, st>>>(dB);
-    k_chunk_scan<<<1, kScanThreads, 0, st>>>(dB);
-    k_chunk_emit<<<gc, kChunkThreads, 0, st>>>(dB);
-    k_emit_rows<<<g, 256, 0, st>>>(dB);
-    k_finish<<<1, 256, 0, st>>>(dB);
+    k_plan<<<1, 1024, 0, st>>>(hB);
+    k_p1<<<p1_grid, kTS, p1_smem, st>>>(hB);
+    k_table_scan<<<g, 256, 0, st>>>(hB);
+    k_chunk_count<<<gc, 256, 0, st>>>(hB);
+    k_chunk_scan<<<1, kScanThreads, 0, st>>>(hB);
+    k_chunk_emit<<<gc, kChunkThreads, 0, st>>>(hB);
+    k_emit_rows<<<g, 256, 0, st>>>(hB);
+    k_finish<<<1, 256, 0, st>>>(hB);
     launches += 8;
     if (cudaGetLastError() != cudaSuccess) return out->status = VFB_DEVICE_ERROR;
   }

@@ -363,24 +363,27 @@ __device__ inline void row_key(const InstDev& I, const uint64_t* row, uint64_t& 
 // ======================================================================= P1
 // Shared per-tile parameters.  s: the stream operand (a row per thread), q:
 // the staged operand (up to kTQ rows, read by every thread).
+__device__ __forceinline__ bool exact_keys(const InstDev& I) { return I.key_mode == KEY_CONCAT && I.lensum <= 126; }
+
 struct __align__(16) TraceSh {
   uint64_t lm;     // length mask
   uint32_t lab, pad;
 };
 struct TileSh {
-  unsigned long long tile;
-  int inst, grp, k, T, TP, half, stride, mode, skip;
+  int inst, k, T, TP, half, stride, mode, skip;
   int kind, mask;   // operand group: 0 unary (bits ~ X F G) / 1 binary (bits & | qUs sUq); the
                     // operators it evaluates
   int otf;          // on-the-fly level: solution test only, nothing inserted
   int nolist;       // new slots are not listed (the table scan reads the whole table)
   int exact;        // every bit of every trace is in the key (KEY_CONCAT, no field cut)
   uint64_t s0, q0, nS, nQ;
-  int si, qi, nq;   // levels of the stream / staged operand; staged rows of this tile
+  int nq;           // staged rows of this tile, or blocks of kTS stream rows of a unary one
+  const uint64_t *srows, *qrows;   // the stream operand's level; this tile's staged rows
+  Slot* tab;
+  uint64_t tmask;
   int qleft;        // the staged operand is the left operand of & | (its index is the major one)
   uint64_t gb[4];   // candidate index of each operator of mask at rows (0, 0)
   // ---- the instance's part (kept while consecutive tiles are of one instance)
-  uint64_t pos[2];  // bit t: trace t is positive
   TraceSh tr[kMaxTraces];    // (the padding word's trace: all zero)
   uint8_t len[kMaxTraces], off[kMaxTraces], wid[kMaxTraces];
   // exact keys: masks over the 126 key bits: every bit; the last step of
@@ -591,10 +594,6 @@ __device__ __forceinline__ void drain_queue(InstDev& I, InsState& S, int keep, P
       }
     }
   }
-}
-
-__device__ __forceinline__ uint64_t pos_bit(const TileSh& P, int t) {
-  return (P.pos[t >> 6] >> (t & 63)) & 1ULL;
 }
 
 // Solution test accumulators: only bit 0 (step 0) of a word is compared
