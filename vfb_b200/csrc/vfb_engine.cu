@@ -117,7 +117,8 @@ struct Engine {
   BatchDev* dB = nullptr;
   InstDev* dInst = nullptr;
   int2* h_status = nullptr;   // pinned mirror of B.status_out
-  unsigned int* h_ctl = nullptr;  // pinned mirror of B.ctl
+  unsigned int* h_ctl = nullptr;  // pinned mirror of B.ctl, then of B.loop_iter
+  unsigned long long* h_iter() { return reinterpret_cast<unsigned long long*>(h_ctl + 4); }
   unsigned long long* d_fail = nullptr;
   uint64_t* h_stage = nullptr;  // pinned upload staging
   size_t h_stage_words = 0;
@@ -130,8 +131,10 @@ struct Engine {
   cudaGraphExec_t exec = nullptr;
   int exec_ninst = -1, exec_smem = -1, exec_grid = -1, exec_loop = -1;
 
-  // device block cache: size -> blocks
-  std::multimap<size_t, void*> free_blocks;
+  // device block cache: size -> blocks (stamp: order of release)
+  struct FreeBlock { void* p; uint64_t stamp; };
+  std::multimap<size_t, FreeBlock> free_blocks;
+  uint64_t release_clock = 0;
   std::map<void*, size_t> live_blocks;
   size_t held_bytes = 0;    // live + cached
   size_t cached_bytes = 0;  // blocks in free_blocks
@@ -213,7 +216,7 @@ struct Engine {
     if (exec) cudaGraphExecDestroy(exec);
     exec = nullptr;
     free_workspace();
-    for (auto& kv : free_blocks) cudaFree(kv.second);
+    for (auto& kv : free_blocks) cudaFree(kv.second.p);
     free_blocks.clear();
     for (auto& kv : live_blocks)
       if (!arena.owns(kv.first)) cudaFree(kv.first);
@@ -289,7 +292,7 @@ struct Engine {
     }
     auto it = free_blocks.lower_bound(bytes);
     if (it != free_blocks.end() && it->first <= 4 * bytes) {
-      void* p = it->second;
+      void* p = it->second.p;
       *got = it->first;
       cached_bytes -= it->first;
       free_blocks.erase(it);
@@ -300,7 +303,7 @@ struct Engine {
     // make room: drop cached blocks before exceeding the budget
     while (mem_limit && held_bytes + bytes > mem_limit && !free_blocks.empty()) {
       auto big = std::prev(free_blocks.end());
-      cudaFreeAsync(big->second, stream);
+      cudaFreeAsync(big->second.p, stream);
       held_bytes -= big->first;
       cached_bytes -= big->first;
       free_blocks.erase(big);
@@ -313,7 +316,7 @@ struct Engine {
       // cached blocks back to the pool and try once more
       if (free_blocks.empty()) return nullptr;
       for (auto& fb : free_blocks) {
-        cudaFreeAsync(fb.second, stream);
+        cudaFreeAsync(fb.second.p, stream);
         held_bytes -= fb.first;
       }
       free_blocks.clear();
@@ -333,14 +336,26 @@ struct Engine {
   // After a call: keep cached at most what the call had live at its peak (the
   // blocks the next call of its kind reuses); the rest, superseded sizes from
   // buffer growth, goes back to the device's memory pool, where other
-  // contexts of the process can allocate it.
+  // contexts of the process can allocate it.  The blocks released longest ago
+  // go first: the call's final buffers, released last, stay.  (Dropping the
+  // largest first made a solve whose rows are 0.4% larger than the last one's
+  // map 6 GB of fresh memory on every call, 38-770 ms against 2.9.)  A call
+  // that came near the budget drops the largest first: a large block kept for
+  // a small request later would be budget that a growth lacks.
   void trim_cache() {
-    while (cached_bytes > peak_live && !free_blocks.empty()) {
-      auto big = std::prev(free_blocks.end());
-      cudaFreeAsync(big->second, stream);
-      held_bytes -= big->first;
-      cached_bytes -= big->first;
-      free_blocks.erase(big);
+    const bool near_limit = mem_limit && peak_live > mem_limit / 3;
+    if (cached_bytes > peak_live) {
+      std::vector<std::multimap<size_t, FreeBlock>::iterator> order;
+      for (auto it = free_blocks.begin(); it != free_blocks.end(); ++it) order.push_back(it);
+      if (near_limit) std::reverse(order.begin(), order.end());
+      else std::sort(order.begin(), order.end(), [](auto x, auto y) { return x->second.stamp < y->second.stamp; });
+      for (auto it : order) {
+        if (cached_bytes <= peak_live) break;
+        cudaFreeAsync(it->second.p, stream);
+        held_bytes -= it->first;
+        cached_bytes -= it->first;
+        free_blocks.erase(it);
+      }
     }
     peak_live = held_bytes - cached_bytes;
   }
@@ -354,7 +369,7 @@ struct Engine {
       live_blocks.erase(it);
       return;
     }
-    free_blocks.emplace(it->second, p);
+    free_blocks.emplace(it->second, FreeBlock{p, ++release_clock});
     cached_bytes += it->second;
     live_blocks.erase(it);
   }
@@ -394,7 +409,7 @@ struct Engine {
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
     if (cudaMalloc(&d_fail, sizeof(unsigned long long)) != cudaSuccess) return VFB_DEVICE_ERROR;
-    if (cudaMallocHost(&h_ctl, 4 * sizeof(unsigned int)) != cudaSuccess) return VFB_DEVICE_ERROR;
+    if (cudaMallocHost(&h_ctl, 6 * sizeof(unsigned int)) != cudaSuccess) return VFB_DEVICE_ERROR;
     if (cudaEventCreate(&ev_t0) != cudaSuccess || cudaEventCreate(&ev_t1) != cudaSuccess) return VFB_DEVICE_ERROR;
     for (auto& e : ev_k)
       if (cudaEventCreate(&e) != cudaSuccess) return VFB_DEVICE_ERROR;
@@ -434,6 +449,18 @@ struct Engine {
       cudaGetLastError();
     }
     return VFB_OK;
+  }
+
+  // P1 CTAs that fill the device at this much dynamic shared memory
+  int p1_occ_smem = -1, p1_occ = 1;
+  int p1_ctas(int smem) {
+    if (smem != p1_occ_smem) {
+      int occ = 1;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, smem);
+      p1_occ = std::max(occ, 1);
+      p1_occ_smem = smem;
+    }
+    return sms * p1_occ;
   }
 
   // ------------------------------------------------------------ workspace
@@ -536,6 +563,19 @@ struct Engine {
     mark();
   }
 
+  // Copies back what the host reads after every launch: the statuses, the
+  // loop's count and, for few instances, their records (their growth and
+  // results then need no copy and wait of their own).
+  static constexpr int kRecordsBack = 4;
+  bool recs_fresh = false;   // h_recs holds what the last launch left
+  bool records_back(int ninst) const { return ninst <= kRecordsBack && h_recs_cap >= ninst; }
+  void copy_back(int ninst, bool loop) {
+    cudaMemcpyAsync(h_status, hB.status_out, (size_t)ninst * sizeof(int2), cudaMemcpyDeviceToHost, stream);
+    if (loop) cudaMemcpyAsync(h_iter(), hB.loop_iter, sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream);
+    if (records_back(ninst))
+      cudaMemcpyAsync(h_recs, dInst, (size_t)ninst * sizeof(InstDev), cudaMemcpyDeviceToHost, stream);
+  }
+
   // Graph: [k_advance, while: (k_p1, k_table_scan_check, k_compact, k_emit, k_advance)] + status
   // read-back, or one step [k_advance, k_p1, ..., k_advance] + status read-back.
   cudaError_t build_graph(int ninst, int p1_smem) {
@@ -581,7 +621,7 @@ struct Engine {
         // status read-back after the loop
         e = cudaStreamBeginCaptureToGraph(stream, graph, &cnode, nullptr, 1, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-          cudaMemcpyAsync(h_status, hB.status_out, (size_t)ninst * sizeof(int2), cudaMemcpyDeviceToHost, stream);
+          copy_back(ninst, true);
           cudaGraph_t out = nullptr;
           e = cudaStreamEndCapture(stream, &out);
         }
@@ -601,7 +641,7 @@ struct Engine {
       e = cudaStreamBeginCaptureToGraph(stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) { cudaGraphDestroy(graph); return e; }
       launch_step(true, profile != 0, p1_smem, 0, false);
-      cudaMemcpyAsync(h_status, hB.status_out, (size_t)ninst * sizeof(int2), cudaMemcpyDeviceToHost, stream);
+      copy_back(ninst, false);
       cudaGraph_t out = nullptr;
       e = cudaStreamEndCapture(stream, &out);
       if (e != cudaSuccess) { cudaGraphDestroy(graph); return e; }
@@ -617,6 +657,7 @@ struct Engine {
   }
 
   cudaError_t run(int ninst, int p1_smem) {
+    recs_fresh = false;
     if (use_coop && !single_step) {
       if (coop_grid <= 0) return cudaErrorInvalidConfiguration;
       const unsigned int init_ctl[2] = {0u, 1u};   // error, continue
@@ -638,8 +679,9 @@ struct Engine {
       const cudaError_t e = build_graph(ninst, p1_smem);
       if (e != cudaSuccess) return e;
     }
-    if (exec_loop) cudaMemsetAsync(hB.loop_iter, 0, sizeof(unsigned long long), stream);
-    c_d2h += (uint64_t)ninst * sizeof(int2);
+    c_d2h += (uint64_t)ninst * sizeof(int2) + (exec_loop ? sizeof(unsigned long long) : 0) +
+             (records_back(ninst) ? (uint64_t)ninst * sizeof(InstDev) : 0);
+    recs_fresh = records_back(ninst);
     return cudaGraphLaunch(exec, stream);
   }
 
@@ -852,15 +894,40 @@ struct Engine {
     return std::max(held, est);
   }
 
-  // cap_bytes > 0: the instance may hold at most that many bytes; a growth
-  // past it ends the instance with VFB_LIMIT.
-  vfb_status grow(InstHost& H, int idx, uint64_t cap_bytes = 0) {
+  // The records of the listed instances into the pinned mirror, one wait for
+  // all of them (none when the last launch brought them back).
+  vfb_status fetch_records(const std::vector<int>& idx, int ninst) {
+    if (idx.empty() || recs_fresh) return VFB_OK;
+    vfb_status s = ensure_recs(ninst);
+    if (s != VFB_OK) return s;
+    for (int i : idx) {
+      if (cudaMemcpyAsync(h_recs + i, dInst + i, sizeof(InstDev), cudaMemcpyDeviceToHost, stream) != cudaSuccess)
+        return dev_fail(__LINE__);
+      c_d2h += sizeof(InstDev);
+    }
+    return cudaStreamSynchronize(stream) == cudaSuccess ? VFB_OK : dev_fail(__LINE__);
+  }
+
+  // Whether every table rehashed since the last call found room for its keys
+  // (they are bounded to half the new table; one wait for all of them).
+  bool rehashed = false;
+  vfb_status check_rehash() {
+    if (!rehashed) return VFB_OK;
+    rehashed = false;
+    unsigned long long fails = 0;
+    cudaMemcpyAsync(&fails, d_fail, sizeof(fails), cudaMemcpyDeviceToHost, stream);
+    c_d2h += sizeof(fails);
+    if (cudaStreamSynchronize(stream) != cudaSuccess || fails) return dev_fail(__LINE__);
+    return VFB_OK;
+  }
+
+  // rec: the instance's record as the device left it.  cap_bytes > 0: the
+  // instance may hold at most that many bytes; a growth past it ends the
+  // instance with VFB_LIMIT.
+  vfb_status grow(InstHost& H, int idx, const InstDev& rec, uint64_t cap_bytes = 0) {
     ++c_grow;
     InstDev& d = H.d;
-    if (cudaMemcpyAsync(&d, dInst + idx, sizeof(InstDev), cudaMemcpyDeviceToHost, stream) != cudaSuccess)
-      return dev_fail(__LINE__);
-    c_d2h += sizeof(InstDev);
-    if (cudaStreamSynchronize(stream) != cudaSuccess) return dev_fail(__LINE__);
+    d = rec;
     const int need = d.need;
     size_t g1, g2;
     if (std::getenv("VFB_DEBUG"))
@@ -939,15 +1006,11 @@ struct Engine {
       if (!pt) return VFB_OOM;
       const uint64_t slots = pow2_at_most(g1 / sizeof(Slot));
       cudaMemsetAsync(pt, 0xFF, slots * sizeof(Slot), stream);
-      cudaMemsetAsync(d_fail, 0, sizeof(unsigned long long), stream);
+      if (!rehashed) cudaMemsetAsync(d_fail, 0, sizeof(unsigned long long), stream);
+      rehashed = true;
       k_rehash<<<grid, 256, 0, stream>>>(d.table, cap, (Slot*)pt, slots - 1, d_fail);
       ++c_launch;
-      unsigned long long fails = 0;
-      cudaMemcpyAsync(&fails, d_fail, sizeof(fails), cudaMemcpyDeviceToHost, stream);
-      c_d2h += sizeof(fails);
-      if (cudaStreamSynchronize(stream) != cudaSuccess) return dev_fail(__LINE__);
-      if (fails) return dev_fail(__LINE__);
-      dfree(d.table);
+      dfree(d.table);   // (handed out again only to work behind the rehash on the stream)
       d.table = (Slot*)pt;
       d.table_mask = slots - 1;
       d.need &= ~NEED_TABLE;
@@ -1056,10 +1119,11 @@ struct Engine {
   // staging buffer, which k_init copies into each level cache (a call of
   // hundreds of instances makes one upload, not one per instance); else each
   // instance's rows go to its level cache directly.
-  vfb_status upload_atoms(const vfb_instance* ins, std::vector<InstHost>& H, int n, bool staged = false) {
+  vfb_status upload_atoms(const vfb_instance* ins, std::vector<InstHost>& H, int n, bool staged = false,
+                          const char* only = nullptr) {
     size_t words = 0;
     for (int i = 0; i < n; ++i)
-      if (H[i].active && H[i].d.rows) words += (size_t)H[i].d.A * H[i].d.TP;
+      if (H[i].active && H[i].d.rows && (!only || only[i])) words += (size_t)H[i].d.A * H[i].d.TP;
     if (words > h_stage_words) {
       if (h_stage) cudaFreeHost(h_stage);
       h_stage = nullptr;
@@ -1069,7 +1133,7 @@ struct Engine {
     }
     size_t o = 0;
     for (int i = 0; i < n; ++i) {
-      if (!H[i].active || !H[i].d.rows) continue;   // (not started yet: no buffers)
+      if (!H[i].active || !H[i].d.rows || (only && !only[i])) continue;   // (not started yet: no buffers)
       const InstDev& d = H[i].d;
       uint64_t* dst = h_stage + o;
       for (int v = 0; v < d.A; ++v) {
@@ -1161,6 +1225,7 @@ struct Engine {
   vfb_status ensure_recs(int n) {
     if (n <= h_recs_cap) return VFB_OK;
     if (cudaStreamSynchronize(stream) != cudaSuccess) return dev_fail(__LINE__);
+    if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }   // (it may copy into the old mirror)
     if (h_recs) cudaFreeHost(h_recs);
     h_recs = nullptr;
     h_recs_cap = 0;
@@ -1191,9 +1256,7 @@ struct Engine {
       maxTP = std::max(maxTP, H[i].d.TP);
     }
     const int p1_smem = p1_smem_bytes(maxTP);
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, p1_smem);
-    p1_grid = sms * std::max(occ, 1);
+    p1_grid = p1_ctas(p1_smem);
     if (use_coop) {
       int occ2 = 0;
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_solve, kTS, p1_smem);
@@ -1261,6 +1324,7 @@ struct Engine {
     }
     int guard = 0;
     bool first = true;
+    recs_fresh = false;
     if (rc == VFB_OK && clusters) {
       rc = run_clusters(H, n, p1_smem);
       first = false;
@@ -1268,7 +1332,11 @@ struct Engine {
     while (rc == VFB_OK) {
       if (!first) {
         bool running = false, grew = false;
-        std::vector<int> waiting;
+        std::vector<int> waiting, asking;
+        for (int i = 0; i < n; ++i)
+          if (H[i].active && (h_status[i].x == ST_NEED_MEM || h_status[i].x == ST_WAIT)) asking.push_back(i);
+        rc = fetch_records(asking, n);
+        if (rc != VFB_OK) break;
         int nrun = 0;
         for (int i = 0; i < n; ++i)
           if (H[i].active && h_status[i].x == ST_RUNNING) ++nrun;
@@ -1277,9 +1345,10 @@ struct Engine {
           const int st = h_status[i].x;
           if (st == ST_RUNNING) running = true;
           if (st == ST_NEED_MEM || st == ST_WAIT) {
-            vfb_status g = grow(H[i], i);
+            // (what a first try did grow is in H[i].d, with what is still asked for)
+            vfb_status g = grow(H[i], i, h_recs[i]);
             // buffers of instances that are done are not needed any more
-            if (g == VFB_OOM && reclaim_finished(H, n)) g = grow(H[i], i);
+            if (g == VFB_OOM && reclaim_finished(H, n)) g = grow(H[i], i, InstDev(H[i].d));
             if (g == VFB_OOM && (nrun > 0 || grew || held_by_others(H, n, i))) {
               // the memory is held by other instances: this one waits (with
               // whatever part did grow) and tries again when the device loop
@@ -1322,6 +1391,7 @@ struct Engine {
           }
           if (st == ST_ERROR) { H[i].fail = VFB_DEVICE_ERROR; H[i].active = false; }
         }
+        if (rc == VFB_OK) rc = check_rehash();
         if (rc != VFB_OK) break;
         const bool pressure = !waiting.empty();
         if (!running && pressure) {
@@ -1352,6 +1422,7 @@ struct Engine {
       }
       first = false;
       cudaError_t e = run(n, p1_smem);
+      if (e == cudaSuccess) e = cudaEventRecord(ev_t1, stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
       if (e != cudaSuccess) { last_error = e; rc = dev_fail(__LINE__); break; }
       if (use_coop) {
@@ -1363,9 +1434,7 @@ struct Engine {
       if (!use_coop && exec_loop) {
         // the plan node, then kBodyLen kernels per loop iteration (each
         // k_advance counts one iteration)
-        unsigned long long it = 0;
-        cudaMemcpy(&it, hB.loop_iter, sizeof(it), cudaMemcpyDeviceToHost);
-        c_d2h += sizeof(it);
+        const unsigned long long it = *h_iter();
         c_launch += it ? 1 + (it - 1) * kBodyLen : 0;
       }
       if (profile) profile_step(n, H);
@@ -1381,13 +1450,15 @@ struct Engine {
       recs_pageable.resize(n);
       recs = recs_pageable.data();
     }
-    if (cudaMemcpyAsync(recs, dInst, (size_t)n * sizeof(InstDev), cudaMemcpyDeviceToHost, stream) !=
-            cudaSuccess) {
-      if (rc == VFB_OK) rc = dev_fail(__LINE__);
+    if (rc != VFB_OK || !recs_fresh) {
+      if (cudaMemcpyAsync(recs, dInst, (size_t)n * sizeof(InstDev), cudaMemcpyDeviceToHost, stream) !=
+              cudaSuccess) {
+        if (rc == VFB_OK) rc = dev_fail(__LINE__);
+      }
+      c_d2h += (uint64_t)n * sizeof(InstDev);
+      cudaEventRecord(ev_t1, stream);
+      if (cudaStreamSynchronize(stream) != cudaSuccess && rc == VFB_OK) rc = dev_fail(__LINE__);
     }
-    c_d2h += (uint64_t)n * sizeof(InstDev);
-    cudaEventRecord(ev_t1, stream);
-    if (cudaStreamSynchronize(stream) != cudaSuccess && rc == VFB_OK) rc = dev_fail(__LINE__);
     float dev_ms = 0;
     cudaEventElapsedTime(&dev_ms, ev_t0, ev_t1);
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1539,7 +1610,6 @@ struct Engine {
     std::vector<int> waited;      // consecutive steps each busy slot has waited for memory
     bool pressure = false;        // some request waited for memory in the last step
     uint64_t evictions = 0;       // requests evicted and queued again (memory held by the others)
-    InstDev* h_inst = nullptr;    // pinned mirror of the slot records
     int p1_smem = 0;
     int tp = 0;                   // row pitch of the most traces a request may have
     double budget_frac = 0.8;     // admission: projected bytes of all slots <= budget_frac * budget
@@ -1579,17 +1649,12 @@ struct Engine {
     sv.request_bytes = sv_request_bytes ? sv_request_bytes : (uint64_t)(mem_limit / 4);
     sv.step_cands = sv_step_cands;
     open_arena();
-    if (cudaMallocHost(&sv.h_inst, (size_t)slots * sizeof(InstDev)) != cudaSuccess) {
-      sv.h_inst = nullptr;
-      return VFB_OOM;
-    }
     const int tp = std::max(2, std::min(max_traces, (int)kMaxTraces) + (max_traces & 1));
     sv.tp = tp;
     sv.p1_smem = p1_smem_bytes(tp);
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, sv.p1_smem);
-    p1_grid = sms * std::max(occ, 1);
+    p1_grid = p1_ctas(sv.p1_smem);
     vfb_status rc = ensure_workspace(slots, (uint64_t)slots * 8);
+    if (rc == VFB_OK) rc = ensure_recs(slots);
     if (rc != VFB_OK) return rc;
     std::vector<InstDev> idle(slots);
     std::memset(idle.data(), 0, idle.size() * sizeof(InstDev));
@@ -1607,7 +1672,7 @@ struct Engine {
   // first, since the arena takes their memory.
   void open_arena() {
     if (arena.base) return;
-    for (auto& kv : free_blocks) cudaFreeAsync(kv.second, stream);
+    for (auto& kv : free_blocks) cudaFreeAsync(kv.second.p, stream);
     free_blocks.clear();
     held_bytes -= cached_bytes;
     cached_bytes = 0;
@@ -1652,7 +1717,6 @@ struct Engine {
   void serve_close() {
     for (int i = 0; i < sv.cap; ++i)
       if (sv.busy[i] && sv.H[i].d.rows) free_buffers(sv.H[i]);
-    if (sv.h_inst) cudaFreeHost(sv.h_inst);
     sv = Session{};
     close_arena();
     trim_cache();
@@ -1713,7 +1777,7 @@ struct Engine {
     if (cudaSetDevice(device) != cudaSuccess) return dev_fail(__LINE__);
     // 1. admission, while the projected bytes of all slots fit the budget;
     // with no slot busy the head of the queue is always admitted
-    bool admitted = false;
+    std::vector<int> admitted;
     uint64_t committed = 0;
     int nbusy = 0;
     for (int i = 0; i < sv.cap; ++i)
@@ -1760,16 +1824,6 @@ struct Engine {
         H.d.promote_above = ~0ULL;
         H.d.p1_quota = sv.step_cands;
       }
-      if (s == VFB_OK) {
-        std::vector<InstHost> one(1);
-        one[0] = H;
-        one[0].active = true;
-        s = upload_atoms(&p.in, one, 1);
-        if (s == VFB_OK &&
-            cudaMemcpyAsync(dInst + i, &H.d, sizeof(InstDev), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-          s = dev_fail(__LINE__);
-        if (s == VFB_OK && cudaStreamSynchronize(stream) != cudaSuccess) s = dev_fail(__LINE__);
-      }
       if (s != VFB_OK) {
         // refused: report it as finished with that status
         if (H.d.rows) free_buffers(H);
@@ -1792,12 +1846,41 @@ struct Engine {
       sv.req[i].in.words = sv.req[i].words.data();
       sv.req[i].in.lengths = sv.req[i].lengths.data();
       sv.queue.pop_front();
-      admitted = true;
+      admitted.push_back(i);
     }
-    if (admitted) {
-      k_fill<<<grid, 256, 0, stream>>>(hB);
-      k_init<<<std::min(sv.cap, grid), 256, 0, stream>>>(hB);
-      c_launch += 2;
+    if (!admitted.empty()) {
+      // their proposition rows in one copy, which k_init spreads, and their
+      // records from the pinned mirror: nothing here is waited for
+      std::vector<vfb_instance> in(sv.cap);
+      for (int i : admitted) in[i] = sv.req[i].in;
+      std::vector<char> is_new(sv.cap, 0);
+      for (int i : admitted) is_new[i] = 1;
+      vfb_status s = upload_atoms(in.data(), sv.H, sv.cap, true, is_new.data());
+      for (int i : admitted) {
+        h_recs[i] = sv.H[i].d;
+        if (s == VFB_OK && cudaMemcpyAsync(dInst + i, h_recs + i, sizeof(InstDev), cudaMemcpyHostToDevice, stream) !=
+                               cudaSuccess)
+          s = dev_fail(__LINE__);
+        c_h2d += sizeof(InstDev);
+      }
+      if (s != VFB_OK) {
+        // refused: reported as finished with that status, as above
+        for (int i : admitted) {
+          cudaMemsetAsync(&dInst[i].status, 0, sizeof(int), stream);   // (ST_IDLE)
+          free_buffers(sv.H[i]);
+          sv.H[i] = InstHost{};
+          sv.busy[i] = 0;
+          if (*ndone >= cap_done) continue;
+          std::memset(&done[*ndone], 0, sizeof(vfb_served));
+          done[*ndone].tag = sv.tag[i];
+          done[*ndone].result.status = s;
+          ++*ndone;
+        }
+      } else {
+        k_fill<<<grid, 256, 0, stream>>>(hB);
+        k_init<<<std::min(sv.cap, grid), 256, 0, stream>>>(hB);
+        c_launch += 2;
+      }
     }
     // 2. one level for every active instance
     int running = 0;
@@ -1824,13 +1907,17 @@ struct Engine {
     // a request that waits alone cannot grow at all and goes on as a solo
     // solve would, its level tested on the fly.  Results stay those of solo
     // solves.
-    std::vector<int> fin, waiting;
+    std::vector<int> fin, waiting, look;
     bool progress = false;
+    for (int i = 0; i < sv.cap; ++i)
+      if (sv.busy[i] && h_status[i].x != ST_RUNNING) look.push_back(i);
+    vfb_status rs = fetch_records(look, sv.cap);
+    if (rs != VFB_OK) return rs;
     for (int i = 0; i < sv.cap; ++i) {
       if (!sv.busy[i]) continue;
       const int st = h_status[i].x;
       if (st == ST_NEED_MEM) {
-        const vfb_status g = grow(sv.H[i], i, sv.request_bytes);
+        const vfb_status g = grow(sv.H[i], i, h_recs[i], sv.request_bytes);
         if (g == VFB_OOM) {
           InstDev& d = sv.H[i].d;
           d.status = ST_NEED_MEM;
@@ -1854,6 +1941,8 @@ struct Engine {
         progress = true;
       }
     }
+    rs = check_rehash();
+    if (rs != VFB_OK) return rs;
     // requests that wait for one another while others keep the device busy
     // (light requests, which free little) are a deadlock too once it lasts
     sv.pressure = !waiting.empty();
@@ -1890,10 +1979,7 @@ struct Engine {
     }
     for (int i : fin) {
       if (*ndone >= cap_done) break;
-      InstDev d;
-      if (cudaMemcpyAsync(&d, dInst + i, sizeof(InstDev), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-          cudaStreamSynchronize(stream) != cudaSuccess)
-        return dev_fail(__LINE__);
+      const InstDev& d = h_recs[i];
       vfb_served& out = done[(*ndone)++];
       out.tag = sv.tag[i];
       slot_result(d, sv.H[i], out.result);
@@ -1904,21 +1990,20 @@ struct Engine {
       free_buffers(sv.H[i]);
       sv.H[i] = InstHost{};
       sv.busy[i] = 0;
-      const int idle = ST_IDLE;
-      cudaMemcpyAsync(&dInst[i].status, &idle, sizeof(int), cudaMemcpyHostToDevice, stream);
+      static_assert(ST_IDLE == 0, "");
+      cudaMemsetAsync(&dInst[i].status, 0, sizeof(int), stream);
     }
     // 5. projections for the next admission (only needed while requests wait)
     int act = 0;
     for (int i = 0; i < sv.cap; ++i) act += sv.busy[i];
     if (act && !sv.queue.empty() && mem_limit) {
-      if (cudaMemcpyAsync(sv.h_inst, dInst, (size_t)sv.cap * sizeof(InstDev), cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess)
-        return dev_fail(__LINE__);
-      if (cudaStreamSynchronize(stream) != cudaSuccess) return dev_fail(__LINE__);
+      std::vector<int> all;
       for (int i = 0; i < sv.cap; ++i)
-        if (sv.busy[i]) sv.proj[i] = projected_bytes(sv.h_inst[i]);
-    } else {
-      cudaStreamSynchronize(stream);
+        if (sv.busy[i]) all.push_back(i);
+      recs_fresh = false;   // (records grown in this step)
+      rs = fetch_records(all, sv.cap);
+      if (rs != VFB_OK) return rs;
+      for (int i : all) sv.proj[i] = projected_bytes(h_recs[i]);
     }
     if (active) *active = act;
     if (queued) *queued = (int)sv.queue.size();

@@ -1335,7 +1335,8 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
   const unsigned long long nchunks = s_carry[1];
   for (unsigned long long c = threadIdx.x; c < nchunks; c += blockDim.x) B.chunk_base[c] = 0;
   if (loop && threadIdx.x == 0) {
-    const unsigned long long it = ++(*B.loop_iter);
+    // (the launch's leading advance starts the count)
+    const unsigned long long it = *B.loop_iter = built ? *B.loop_iter + 1 : 1;
     const bool more = s_run && !s_need && it < max_iter;
     cudaGraphSetConditional(handle, more ? 1u : 0u);
   }
