@@ -59,16 +59,16 @@ __global__ void k_bs_level(BsDev D, int c, unsigned long long cands) {
 }
 
 // Owner bits: a slot whose payload carries level c (0: base) marks its index
-// when the index is below limit.
+// when the index is below limit and the size's solving candidate (an empty
+// slot's payload carries no level).
 __global__ void k_bs_mark(BsDev D, int c, unsigned long long cap, unsigned long long limit) {
+  const unsigned long long best = __ldcg(D.best), lim = best < limit ? best : limit;
   for (unsigned long long s = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; s < cap;
        s += (unsigned long long)gridDim.x * blockDim.x) {
-    const Key128 k = ld_key(D.tab + s);
-    if (k.h == kEmpty && k.l == kEmpty) continue;
     const unsigned long long pay = __ldcg(&D.tab[s].pay);
     if ((pay >> kPayShift) != (unsigned long long)c) continue;
     const uint64_t g = pay & kIdxMask;
-    if (g < limit) atomicOr(D.bitmap + (g >> 5), 1u << (g & 31));
+    if (g < lim) atomicOr(D.bitmap + (g >> 5), 1u << (g & 31));
   }
 }
 
@@ -84,10 +84,27 @@ __global__ void k_bs_count(BsDev D, unsigned long long nwords) {
   if (threadIdx.x == 0) D.counts[blockIdx.x] = tot;
 }
 
-// Owners of each chunk appended in order from entry out0 + offs[chunk]: their
-// words and their indices (cache row for base entries, candidate index else);
-// the chunk's bitmap words are cleared.
-__global__ void k_bs_emit(BsDev D, int c, unsigned long long nwords, unsigned long long out0) {
+// Exclusive prefix of the chunks' counts and their total (one CTA).
+__global__ void __launch_bounds__(1024) k_bs_offsets(BsDev D, unsigned chunks) {
+  __shared__ unsigned long long s_w[32];
+  unsigned long long run = 0;
+  for (unsigned c0 = 0; c0 < chunks; c0 += blockDim.x) {
+    const unsigned c = c0 + threadIdx.x;
+    const unsigned long long v = c < chunks ? D.counts[c] : 0ULL;
+    unsigned long long tot;
+    const unsigned long long ex = block_excl_scan(v, s_w, tot);
+    if (c < chunks) D.offs[c] = run + ex;
+    run += tot;
+  }
+  if (threadIdx.x == 0) *D.total = run;
+}
+
+// Owners of each chunk listed in order from entry out0 + offs[chunk] (cache
+// row for base entries, candidate index else); the chunk's bitmap words are
+// cleared.  Their words are a kernel of their own (k_bs_vals), a thread per
+// entry: decoded here, one thread after another through the up to 128 owners
+// of its bitmap words, they took 110-205 us a size.
+__global__ void k_bs_emit(BsDev D, unsigned long long nwords, unsigned long long out0) {
   __shared__ unsigned long long s_w[32];
   constexpr int kPer = kBsChunkWords / 256;
   const unsigned long long w0 = (unsigned long long)blockIdx.x * kBsChunkWords + (unsigned long long)threadIdx.x * kPer;
@@ -104,31 +121,27 @@ __global__ void k_bs_emit(BsDev D, int c, unsigned long long nwords, unsigned lo
   for (int u = 0; u < kPer; ++u) {
     uint32_t b = bits[u];
     if (b) D.bitmap[w0 + u] = 0u;
-    while (b) {
-      const int bit = __ffs(b) - 1;
-      b &= b - 1;
-      const uint64_t g = (w0 + u) * 32 + bit;
-      uint64_t v;
-      if (c == 0) {
-        v = bs_project(D, g);
-      } else {
-        v = bs_value(D, bs_decode(D.st, D.cn, c, g));
-      }
-      D.vals[pos] = v;
-      D.org[pos] = g;
-      ++pos;
-    }
+    for (; b; b &= b - 1) D.org[pos++] = (w0 + u) * 32 + __ffs(b) - 1;
+  }
+}
+
+// The words of the size's entries (c = 0: base).
+__global__ void k_bs_vals(BsDev D, int c, unsigned long long out0) {
+  const unsigned long long n = *D.total;
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (unsigned long long)gridDim.x * blockDim.x) {
+    const uint64_t g = D.org[out0 + i];
+    D.vals[out0 + i] = c == 0 ? bs_project(D, g) : bs_value(D, bs_decode(D.st, D.cn, c, g));
   }
 }
 
 // First entry index at or after each of n row boundaries (entries ascending by
 // row): the base sizes' start entries.
-__global__ void k_bs_bounds(BsDev D, unsigned long long nent, const unsigned long long* rows_at, int n,
-                            unsigned long long* out) {
+__global__ void k_bs_bounds(BsDev D, const unsigned long long* rows_at, int n, unsigned long long* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned long long x = rows_at[i];
-  unsigned long long lo = 0, hi = nent;
+  unsigned long long lo = 0, hi = *D.total;
   while (lo < hi) {
     const unsigned long long mid = (lo + hi) >> 1;
     if (__ldcg(D.org + mid) < x) lo = mid + 1; else hi = mid;

@@ -2059,6 +2059,7 @@ struct Engine {
     D.offs = (unsigned long long*)take(chunk_cap * 8);
     D.best = (unsigned long long*)take(64);
     D.fail = D.best + 1;
+    D.total = D.best + 2;
     unsigned long long* bnd = (unsigned long long*)take(2 * (kMaxSize + 2) * 8);
     if (!D.tab || !D.vals || !D.org || !D.bitmap || !D.counts || !D.offs || !D.best || !bnd) {
       release();
@@ -2070,49 +2071,44 @@ struct Engine {
     cudaMemsetAsync(D.best, 0xFF, 8, stream);
     cudaMemsetAsync(D.fail, 0, 8, stream);
     const int g256 = sms * 8;
-    std::vector<unsigned long long> hcount;
-    // compaction of the owner bits below nbits into entries from out0
-    auto compact = [&](int c, uint64_t nbits, uint64_t out0, uint64_t& n_out) -> vfb_status {
+    // compaction of the owner bits below nbits into entries from out0 (there is
+    // room for every one of them); their number is left in D.total
+    auto compact = [&](int c, uint64_t nbits, uint64_t out0) {
       const uint64_t nwords = (nbits + 31) / 32;
       const unsigned chunks = (unsigned)((nwords + kBsChunkWords - 1) / kBsChunkWords);
-      if (chunks == 0) { n_out = 0; return VFB_OK; }
-      k_bs_count<<<chunks, 256, 0, stream>>>(D, (unsigned long long)nwords);
-      hcount.assign(chunks, 0);
-      if (cudaMemcpyAsync(hcount.data(), D.counts, chunks * 8, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-          cudaStreamSynchronize(stream) != cudaSuccess)
-        return dev_fail(__LINE__);
-      unsigned long long run = 0;
-      for (unsigned j = 0; j < chunks; ++j) { const unsigned long long x = hcount[j]; hcount[j] = run; run += x; }
-      if (out0 + run > ent_cap) return VFB_OOM;
-      cudaMemcpyAsync(D.offs, hcount.data(), chunks * 8, cudaMemcpyHostToDevice, stream);
-      k_bs_emit<<<chunks, 256, 0, stream>>>(D, c, (unsigned long long)nwords, (unsigned long long)out0);
-      c_launch += 2;
-      n_out = run;
-      return VFB_OK;
+      if (chunks) k_bs_count<<<chunks, 256, 0, stream>>>(D, (unsigned long long)nwords);
+      k_bs_offsets<<<1, 1024, 0, stream>>>(D, chunks);
+      if (chunks) k_bs_emit<<<chunks, 256, 0, stream>>>(D, (unsigned long long)nwords, (unsigned long long)out0);
+      k_bs_vals<<<g256, 256, 0, stream>>>(D, c, (unsigned long long)out0);
+      c_launch += chunks ? 4 : 2;
+    };
+    // the size's solving candidate, probe failures and entries
+    unsigned long long got[3] = {~0ULL, 0, 0};
+    auto read_back = [&]() {
+      cudaMemcpyAsync(got, D.best, sizeof(got), cudaMemcpyDeviceToHost, stream);
+      return cudaStreamSynchronize(stream) == cudaSuccess ? VFB_OK : dev_fail(__LINE__);
     };
     // base entries: the rows' words, first occurrence in row order
     k_bs_base<<<g256, 256, 0, stream>>>(D, (unsigned long long)nrows);
     k_bs_mark<<<g256, 256, 0, stream>>>(D, 0, (unsigned long long)slots, (unsigned long long)nrows);
     c_launch += 2;
-    uint64_t nent = 0;
-    rc = compact(0, nrows, 0, nent);
-    unsigned long long fails = 0;
-    if (rc == VFB_OK) {
+    compact(0, nrows, 0);
+    {
       std::vector<unsigned long long> at(K + 1), pos(K + 1);
       for (int c = 1; c <= K; ++c) at[c - 1] = d.lstart[c];
       at[K] = nrows;
       cudaMemcpyAsync(bnd, at.data(), (K + 1) * 8, cudaMemcpyHostToDevice, stream);
-      k_bs_bounds<<<1, 64, 0, stream>>>(D, (unsigned long long)nent, bnd, K + 1, bnd + kMaxSize + 2);
+      k_bs_bounds<<<1, 64, 0, stream>>>(D, bnd, K + 1, bnd + kMaxSize + 2);
       ++c_launch;
       cudaMemcpyAsync(pos.data(), bnd + kMaxSize + 2, (K + 1) * 8, cudaMemcpyDeviceToHost, stream);
-      cudaMemcpyAsync(&fails, D.fail, 8, cudaMemcpyDeviceToHost, stream);
-      if (cudaStreamSynchronize(stream) != cudaSuccess) rc = dev_fail(__LINE__);
+      rc = read_back();
       for (int c = 1; c <= K; ++c) {
         D.st[c] = pos[c - 1];
         D.cn[c] = pos[c] - pos[c - 1];
       }
     }
-    if (rc == VFB_OK && fails) rc = VFB_LIMIT;
+    uint64_t nent = got[2];
+    if (rc == VFB_OK && got[1]) rc = VFB_LIMIT;
     uint64_t total_bs = 0;
     unsigned long long best = ~0ULL;
     int c = K;
@@ -2174,20 +2170,18 @@ struct Engine {
         words_cap = nw;
         chunk_cap = ncap;
       }
+      // (the owners are listed before the host knows whether a candidate
+      // solves: only those below it are marked, and every candidate has room)
       cudaMemsetAsync(D.best, 0xFF, 8, stream);
       k_bs_level<<<g256, 256, 0, stream>>>(D, c, (unsigned long long)nc);
-      ++c_launch;
-      cudaMemcpyAsync(&best, D.best, 8, cudaMemcpyDeviceToHost, stream);
-      cudaMemcpyAsync(&fails, D.fail, 8, cudaMemcpyDeviceToHost, stream);
-      if (cudaStreamSynchronize(stream) != cudaSuccess) { rc = dev_fail(__LINE__); break; }
-      if (fails) { rc = VFB_LIMIT; break; }
-      // new entries: the owners (below the solving candidate, if any)
-      const uint64_t lim = best != ~0ULL ? best : nc;
-      k_bs_mark<<<g256, 256, 0, stream>>>(D, c, (unsigned long long)slots, (unsigned long long)lim);
-      ++c_launch;
-      uint64_t nnew = 0;
-      rc = compact(c, lim, nent, nnew);
+      k_bs_mark<<<g256, 256, 0, stream>>>(D, c, (unsigned long long)slots, (unsigned long long)nc);
+      c_launch += 2;
+      compact(c, nc, nent);
+      rc = read_back();
       if (rc != VFB_OK) break;
+      best = got[0];
+      if (got[1]) { rc = VFB_LIMIT; break; }
+      const uint64_t nnew = got[2];
       D.st[c] = nent;
       D.cn[c] = nnew;
       nent += nnew;

@@ -131,6 +131,7 @@ struct BsDev {
   unsigned long long* offs;        // chunk offsets (exclusive prefix of counts)
   unsigned long long* best;        // first solving candidate of the size
   unsigned long long* fail;        // probe failures
+  unsigned long long* total;       // owners of the size
   uint64_t st[kMaxSize + 2], cn[kMaxSize + 2];   // first entry and entries of each size
 };
 struct BsCand {
@@ -159,9 +160,10 @@ __global__ void k_bs_base(BsDev D, unsigned long long nrows);
 __global__ void k_bs_level(BsDev D, int c, unsigned long long cands);
 __global__ void k_bs_mark(BsDev D, int c, unsigned long long cap, unsigned long long limit);
 __global__ void k_bs_count(BsDev D, unsigned long long nwords);
-__global__ void k_bs_emit(BsDev D, int c, unsigned long long nwords, unsigned long long out0);
-__global__ void k_bs_bounds(BsDev D, unsigned long long nent, const unsigned long long* rows_at, int n,
-                            unsigned long long* out);
+__global__ void k_bs_offsets(BsDev D, unsigned chunks);
+__global__ void k_bs_emit(BsDev D, unsigned long long nwords, unsigned long long out0);
+__global__ void k_bs_vals(BsDev D, int c, unsigned long long out0);
+__global__ void k_bs_bounds(BsDev D, const unsigned long long* rows_at, int n, unsigned long long* out);
 __global__ void k_bs_leaves(const InstDev* I, const unsigned long long* rows, int n, int16_t* rpn, int* len);
 
 // Set-up and maintenance kernels.
