@@ -2282,6 +2282,7 @@ struct Engine {
   // first solution of the numbering.  Sizes whose count passes 2^62 end the
   // search with VFB_LIMIT.
   static constexpr unsigned long long kExhRange = 1ull << 28;
+  static constexpr unsigned long long kExhAhead = 1ull << 16;   // formulas launched without a look at the results
 
   static void exh_decode_host(uint64_t n, int k, const uint64_t (*cnt)[8], int16_t* rpn) {
     if (k == 1) { rpn[0] = (int16_t)n; return; }
@@ -2348,43 +2349,72 @@ struct Engine {
     }
     for (int i = 1; i <= kfit; ++i)
       for (int o = 0; o < 8; ++o) h.cnt[i][o] = (uint64_t)c[i][o];
-    size_t g1 = 0, g2 = 0;
+    size_t g1 = 0, g2 = 0, g3 = 0;
     void* pd = dalloc(sizeof(ExhDev), &g1);
-    void* pb = pd ? dalloc(sizeof(unsigned long long), &g2) : nullptr;
+    void* pb = pd ? dalloc((kMaxSize + 2) * sizeof(unsigned long long), &g2) : nullptr;
+    // the table of the small sizes' words: as many sizes as fit its bound, and
+    // the memory; the propositions at least, whose words the record holds anyway
+    h.m = 1;
+    h.entries = (uint64_t)A;
+    while (h.m < kfit && h.cnt[h.m + 1][7] <= kExhTableWords && (h.entries + h.cnt[h.m + 1][7]) * T <= kExhTableWords)
+      h.entries += h.cnt[++h.m][7];
+    void* pt = pb ? dalloc(h.entries * T * 8, &g3) : nullptr;
+    while (pb && !pt && h.m > 1) {
+      h.entries -= h.cnt[h.m--][7];
+      pt = dalloc(h.entries * T * 8, &g3);
+    }
     if (!pd || !pb) { dfree(pd); return r.status = VFB_OOM; }
+    h.tab = pt ? (uint64_t*)pt : ((ExhDev*)pd)->words;
+    for (int k = 2; k <= h.m; ++k) h.first[k] = h.first[k - 1] + h.cnt[k - 1][7];
     ExhDev* dP = (ExhDev*)pd;
     unsigned long long* dBest = (unsigned long long*)pb;
     cudaEventRecord(ev_t0, stream);
     vfb_status rc = VFB_OK;
     if (cudaMemcpyAsync(dP, &h, sizeof(ExhDev), cudaMemcpyHostToDevice, stream) != cudaSuccess ||
-        cudaMemsetAsync(dBest, 0xFF, sizeof(unsigned long long), stream) != cudaSuccess)
+        cudaMemsetAsync(dBest, 0xFF, (kMaxSize + 2) * sizeof(unsigned long long), stream) != cudaSuccess)
       rc = dev_fail(__LINE__);
     c_h2d += sizeof(ExhDev);
-    unsigned long long best = ~0ULL;
+    unsigned long long best[kMaxSize + 2];
     int found_k = 0;
+    // small sizes are launched without waiting for the ones before them (a
+    // size whose smaller ones have a solution ends at once); the host looks
+    // after kExhAhead formulas, and after every range of a larger size
+    unsigned long long ahead = 0;
+    int looked = 0;   // sizes known to have no solution
     for (int k = 1; k <= kfit && rc == VFB_OK && !found_k; ++k) {
       const unsigned long long total = h.cnt[k][7];
-      for (unsigned long long lo = 0; lo < total; lo += kExhRange) {
-        const unsigned long long hi = std::min(total, lo + kExhRange);
-        const unsigned long long nthreads = hi - lo;
-        const unsigned blocks = (unsigned)std::min<unsigned long long>((nthreads + 255) / 256,
+      unsigned long long hi = total;
+      for (unsigned long long lo = 0; lo < total && rc == VFB_OK && !found_k; lo = hi) {
+        hi = std::min(total, lo + kExhRange);
+        const unsigned blocks = (unsigned)std::min<unsigned long long>((hi - lo + 255) / 256,
                                                                        (unsigned long long)sms * 16);
-        k_exhaustive<<<blocks, 256, 0, stream>>>(dP, k, lo, hi, dBest);
+        if (k <= h.m) {
+          k_exh_table<<<blocks, 256, 0, stream>>>(dP, k, dBest);
+          hi = total;
+        } else {
+          k_exhaustive<<<blocks, 256, 0, stream>>>(dP, k, lo, hi, dBest);
+        }
         ++c_launch;
-        if (cudaMemcpyAsync(&best, dBest, sizeof(best), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+        ahead += hi - lo;
+        r.level_cands[k] = hi;
+        if (k < kfit && hi == total && ahead + h.cnt[k + 1][7] <= kExhAhead) continue;
+        if (cudaMemcpyAsync(best, dBest, sizeof(best), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
           rc = dev_fail(__LINE__);
           break;
         }
         c_d2h += sizeof(best);
-        if (best != ~0ULL) {
-          r.level_cands[k] = best + 1;
-          found_k = k;
-          break;
-        }
-        r.level_cands[k] = hi;
+        ahead = 0;
+        for (int q = looked + 1; q <= k && !found_k; ++q)
+          if (best[q] != ~0ULL) found_k = q;
+        looked = hi == total ? k : k - 1;
       }
       r.size = k;
+    }
+    if (found_k) {
+      // (sizes launched past it found nothing to do)
+      for (int q = found_k + 1; q <= kMaxSize; ++q) r.level_cands[q] = 0;
+      r.level_cands[found_k] = best[found_k] + 1;
     }
     cudaEventRecord(ev_t1, stream);
     cudaStreamSynchronize(stream);
@@ -2392,6 +2422,7 @@ struct Engine {
     cudaEventElapsedTime(&ms, ev_t0, ev_t1);
     dfree(pd);
     dfree(pb);
+    dfree(pt);
     if (rc != VFB_OK) return r.status = rc;
     r.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     r.device_seconds = ms * 1e-3;
@@ -2399,9 +2430,9 @@ struct Engine {
     r.d2h_bytes = c_d2h;
     r.kernel_launches = c_launch;
     if (found_k) {
-      exh_decode_host(best, found_k, h.cnt, r.rpn);
+      exh_decode_host(best[found_k], found_k, h.cnt, r.rpn);
       r.rpn_len = found_k;
-      r.solution_index = best;
+      r.solution_index = best[found_k];
       r.size = found_k;
       return r.status = VFB_OK;
     }

@@ -102,16 +102,21 @@ struct ClusterWork {
 };
 __global__ void k_cluster(ClusterWork W);
 
-// Cache-free search (vfb_exhaustive.cu): the instance and the count matrix
-// of the formula numbering; formula numbers [lo, hi) of size k are evaluated
-// and the smallest solving number lowers *best.
+// Cache-free search (vfb_exhaustive.cu): the instance, the count matrix of
+// the formula numbering, and the table of the words of all formulas of sizes
+// 1..m: tab[t * entries + first[s] + n] = formula n of size s on trace t.
+constexpr uint64_t kExhTableWords = 1ull << 20;
 struct ExhDev {
-  int A, T;
+  int A, T, m;
+  uint64_t entries;
+  uint64_t* tab;
+  uint64_t first[kMaxSize + 1];    // first[0] unused
   uint64_t cnt[kMaxSize + 1][8];   // formulas per size and root operator (7: all of the size)
   uint64_t posmask[2];             // bit t: trace t is positive
   uint8_t len[kMaxTraces];
   uint64_t words[kMaxTraces * 64]; // words[t * A + v]: proposition v on trace t
 };
+__global__ void k_exh_table(const ExhDev* P, int k, unsigned long long* best);
 __global__ void k_exhaustive(const ExhDev* P, int k, unsigned long long lo, unsigned long long hi,
                              unsigned long long* best);
 
