@@ -556,12 +556,11 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
 }
 
 // CTA bid of nb: its first tile is tile bid, the later ones come by ticket.
-__device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb) {
+__device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb, unsigned long long total) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ TileSh P;
   __shared__ WarpIns s_ins[kTS / 32];
   __shared__ unsigned long long s_red[3][kTS / 32], s_next;
-  const unsigned long long total = B.p1_prefix[B.ninst];
   InsState S{&s_ins[threadIdx.x >> 5], nullptr, 0, 0, 0, false};
   QKey* sK = reinterpret_cast<QKey*>(smem);
   QWord* sQ = reinterpret_cast<QWord*>(smem) + kTQ;
@@ -682,9 +681,10 @@ __device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb) {
 
 __global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev B) {
   step_entry();
-  const unsigned long long cap = B.tickets[kTicketP1Blocks];   // the tuned CTA count of this step
+  // the tuned CTA count of this step and its tiles (read together)
+  const unsigned long long cap = __ldcg(B.tickets + kTicketP1Blocks), total = __ldcg(B.p1_prefix + B.ninst);
   const unsigned nb = cap && cap < gridDim.x ? (unsigned)cap : gridDim.x;
-  if (blockIdx.x < nb) ph_p1(B, blockIdx.x, nb);
+  if (blockIdx.x < nb) ph_p1(B, blockIdx.x, nb, total);
 }
 
 // ============================================================== table scan
@@ -1642,7 +1642,7 @@ __global__ void __launch_bounds__(kTS) k_solve(BatchDev* Bp, unsigned int max_st
     if (!grid_sync(ctl, nb)) return;
     if (bid == 0 && threadIdx.x == 0) ph_plan_prefix(B);
     if (!grid_sync(ctl, nb)) return;
-    ph_p1(B, bid, nb);
+    ph_p1(B, bid, nb, B.p1_prefix[B.ninst]);
     if (!grid_sync(ctl, nb)) return;
     ph_table_scan(B, bid, nb);
     if (!grid_sync(ctl, nb)) return;
@@ -1705,7 +1705,7 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
       cl.sync();
       if (rank == 0 && threadIdx.x == 0) ph_plan_prefix(B);
       cl.sync();
-      ph_p1(B, rank, csize);
+      ph_p1(B, rank, csize, B.p1_prefix[1]);
       cl.sync();
       ph_table_scan(B, rank, csize);
       cl.sync();
@@ -1726,24 +1726,43 @@ __global__ void __launch_bounds__(kTS) k_cluster(ClusterWork W) {
 // ==================================================================== fill
 // First buffers of new instances (fill set by the host): empty table (every
 // word ~0) and clear owner bitmap, every thread of the grid on one instance
-// after the other.
+// after the other.  A warp reads the records of 32 instances at once, a lane
+// each (one after the other, a batch of 256 waited 0.3 ms for its loads).
 __global__ void k_fill(const __grid_constant__ BatchDev B) {
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-  for (int b = 0; b < B.ninst; ++b) {
-    const InstDev& I = B.inst[b];
-    if (!I.fill || I.status != ST_RUNNING || I.level != 1) continue;
-    ulonglong2* tab = reinterpret_cast<ulonglong2*>(I.table);
-    const uint64_t nt = (I.table_mask + 1) * (sizeof(Slot) / sizeof(ulonglong2));
-    for (uint64_t x = tid; x < nt; x += nth) tab[x] = make_ulonglong2(~0ULL, ~0ULL);
-    for (uint64_t x = tid; x < I.bitmap_words; x += nth) I.bitmap[x] = 0u;
+  const int lane = threadIdx.x & 31;
+  for (int b0 = 0; b0 < B.ninst; b0 += 32) {
+    const int b = b0 + lane;
+    bool mine = false;
+    unsigned long long table = 0, slots = 0, bitmap = 0, words = 0;
+    if (b < B.ninst) {
+      const InstDev& I = B.inst[b];
+      mine = I.fill && I.status == ST_RUNNING && I.level == 1;
+      table = (unsigned long long)I.table;
+      slots = I.table_mask + 1;
+      bitmap = (unsigned long long)I.bitmap;
+      words = I.bitmap_words;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, mine); m; m &= m - 1) {
+      const int j = __ffs(m) - 1;
+      ulonglong2* tab = (ulonglong2*)__shfl_sync(0xffffffffu, table, j);
+      const uint64_t nt = __shfl_sync(0xffffffffu, slots, j) * (sizeof(Slot) / sizeof(ulonglong2));
+      uint32_t* bits = (uint32_t*)__shfl_sync(0xffffffffu, bitmap, j);
+      const uint64_t nb = __shfl_sync(0xffffffffu, words, j);
+      for (uint64_t x = tid; x < nt; x += nth) tab[x] = make_ulonglong2(~0ULL, ~0ULL);
+      for (uint64_t x = tid; x < nb; x += nth) bits[x] = 0u;
+    }
   }
 }
 
 // ==================================================================== init
 // Level 1: every proposition is a row (duplicates included); its key enters
 // the set; propositions are tested as size-1 solutions in order
-// (LTL_BS.cu:1127-1163, hashSetsInitialisation 136-160).
+// (LTL_BS.cu:1127-1163, hashSetsInitialisation 136-160).  A warp per
+// proposition, a lane per trace word: a thread per proposition walked its
+// row word by word, one load after another (6.1 us against 4.9 for a few short
+// traces, 45 against 16 for 128).
 __global__ void k_init(const __grid_constant__ BatchDev B) {
   __shared__ unsigned long long s_first;
   __shared__ unsigned long long s_new;
@@ -1755,36 +1774,54 @@ __global__ void k_init(const __grid_constant__ BatchDev B) {
       s_new = 0;
       for (int o = 0; o < 4; ++o) I.uhit[atom_level(I)][o] = 0u;
     }
-    if (I.atoms_staged) {
-      if (!B.atoms) {   // (never: the host uploads them before this launch)
-        __syncthreads();
-        if (threadIdx.x == 0) I.status = ST_ERROR;
-        continue;
-      }
-      const uint64_t nw = (uint64_t)I.A * I.TP;
-      for (uint64_t w = threadIdx.x; w < nw; w += blockDim.x) I.rows[w] = B.atoms[I.atom_off + w];
+    const bool staged = I.atoms_staged;
+    if (staged && !B.atoms) {   // (never: the host uploads them before this launch)
+      __syncthreads();
+      if (threadIdx.x == 0) I.status = ST_ERROR;
+      continue;
     }
     __syncthreads();
-    for (int v = threadIdx.x; v < I.A; v += blockDim.x) {
-      const uint64_t* row = I.rows + (uint64_t)v * I.TP;
-      uint64_t h, l;
-      row_key(I, row, h, l);
-      int isnew = 0;
-      uint64_t idx = slot_hash(h, l) & I.table_mask;
-      const int r = insert_min(I.table, I.table_mask, idx, ld_key(I.table + idx), h, l,
-                               pay_of(atom_level(I), v), isnew);
-      if (r < 0) atomicAdd(&I.probe_fail, 1ULL);
-      if (isnew) atomicAdd(&s_new, 1ULL);
-      I.origin[v] = v;
+    const int lane = threadIdx.x & 31, T = I.T, TP = I.TP, half = T / 2, mode = I.key_mode;
+    for (int v = threadIdx.x >> 5; v < I.A; v += blockDim.x >> 5) {
+      uint64_t* row = I.rows + (uint64_t)v * TP;
+      const uint64_t* from = staged ? B.atoms + I.atom_off + (uint64_t)v * TP : row;
+      KeyAcc k;
+      key_init(k);
       bool sol = true;
       unsigned miss = 0u;
-      for (int t = 0; t < I.T; ++t) {
+      for (int t = lane; t < TP; t += 32) {
+        const uint64_t w = from[t];
+        if (staged) row[t] = w;
+        if (t >= T) continue;
+        const int L = I.len[t];
         const unsigned lab = is_pos(I, t) ? 1u : 0u;
-        sol = sol && (((row[t] & 1ULL) != 0) == (lab != 0));
-        miss |= unary_miss(row[t], len_mask(I.len[t]), lab);
+        sol = sol && (((w & 1ULL) != 0) == (lab != 0));
+        miss |= unary_miss(w, len_mask(L), lab);
+        if (mode == KEY_HASH) key_word<KEY_HASH>(k, w, t, half, 0, 0, 0, 0);
+        else if (mode == KEY_SAMPLED) key_word<KEY_SAMPLED>(k, w, t, half, I.off[t], I.width[t], I.stride1, L);
+        else key_word<KEY_CONCAT>(k, w, t, half, I.off[t], I.width[t], 0, L);
       }
-      if (sol) atomicMin(&s_first, (unsigned long long)v);
-      record_unary(I, atom_level(I), (uint64_t)v, miss);
+      sol = __all_sync(0xffffffffu, sol);
+      miss = __reduce_or_sync(0xffffffffu, miss);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        k.a0 ^= __shfl_xor_sync(0xffffffffu, k.a0, o);
+        k.a1 ^= __shfl_xor_sync(0xffffffffu, k.a1, o);
+      }
+      if (lane == 0) {
+        uint64_t h, l;
+        if (mode == KEY_HASH) key_final<KEY_HASH>(k, h, l);
+        else key_final<KEY_CONCAT>(k, h, l);   // (the bit-field modes end alike)
+        int isnew = 0;
+        uint64_t idx = slot_hash(h, l) & I.table_mask;
+        const int r = insert_min(I.table, I.table_mask, idx, ld_key(I.table + idx), h, l,
+                                 pay_of(atom_level(I), v), isnew);
+        if (r < 0) atomicAdd(&I.probe_fail, 1ULL);
+        if (isnew) atomicAdd(&s_new, 1ULL);
+        I.origin[v] = v;
+        if (sol) atomicMin(&s_first, (unsigned long long)v);
+        record_unary(I, atom_level(I), (uint64_t)v, miss);
+      }
     }
     __syncthreads();
     if (threadIdx.x == 0) {

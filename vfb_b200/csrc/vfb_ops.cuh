@@ -339,27 +339,6 @@ __device__ inline void cand_key(const InstDev& I, const Cand& c, uint64_t& h, ui
   key_final<MODE>(k, h, l);
 }
 
-__device__ inline void row_key(const InstDev& I, const uint64_t* row, uint64_t& h, uint64_t& l) {
-  KeyAcc k;
-  key_init(k);
-  const int T = I.T, half = T / 2;
-  switch (I.key_mode) {
-    case KEY_HASH:
-      for (int t = 0; t < T; ++t) key_word<KEY_HASH>(k, row[t], t, half, 0, 0, 0, 0);
-      key_final<KEY_HASH>(k, h, l);
-      break;
-    case KEY_SAMPLED:
-      for (int t = 0; t < T; ++t)
-        key_word<KEY_SAMPLED>(k, row[t], t, half, I.off[t], I.width[t], I.stride1, I.len[t]);
-      key_final<KEY_SAMPLED>(k, h, l);
-      break;
-    default:
-      for (int t = 0; t < T; ++t)
-        key_word<KEY_CONCAT>(k, row[t], t, half, I.off[t], I.width[t], 0, I.len[t]);
-      key_final<KEY_CONCAT>(k, h, l);
-  }
-}
-
 // ======================================================================= P1
 // Shared per-tile parameters.  s: the stream operand (a row per thread), q:
 // the staged operand (up to kTQ rows, read by every thread).
