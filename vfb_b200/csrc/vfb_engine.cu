@@ -334,23 +334,26 @@ struct Engine {
   }
 
   // After a call: keep cached at most what the call had live at its peak (the
-  // blocks the next call of its kind reuses); the rest, superseded sizes from
-  // buffer growth, goes back to the device's memory pool, where other
-  // contexts of the process can allocate it.  The blocks released longest ago
-  // go first: the call's final buffers, released last, stay.  (Dropping the
-  // largest first made a solve whose rows are 0.4% larger than the last one's
-  // map 6 GB of fresh memory on every call, 38-770 ms against 2.9.)  A call
-  // that came near the budget drops the largest first: a large block kept for
-  // a small request later would be budget that a growth lacks.
+  // blocks the next call of its kind reuses), or an eighth of the budget where
+  // that is more (calls in turn whose needs differ); the rest goes back to the
+  // device's memory pool, where other contexts of the process can allocate it.
+  // The blocks released longest ago go first: the call's final buffers,
+  // released last, stay.  (Dropping the largest first, down to the call's peak,
+  // made a solve whose rows are 0.4% larger than the last one's map 6 GB of
+  // fresh memory on every call, 38-770 ms against 2.9; batches in turn 7.5-15
+  // ms against 5.)  A call that came near the budget keeps its peak and drops
+  // the largest first: a large block kept for a small request later would be
+  // budget that a growth lacks.
   void trim_cache() {
     const bool near_limit = mem_limit && peak_live > mem_limit / 3;
-    if (cached_bytes > peak_live) {
+    const size_t keep = near_limit ? peak_live : std::max(peak_live, mem_limit / 8);
+    if (cached_bytes > keep) {
       std::vector<std::multimap<size_t, FreeBlock>::iterator> order;
       for (auto it = free_blocks.begin(); it != free_blocks.end(); ++it) order.push_back(it);
       if (near_limit) std::reverse(order.begin(), order.end());
       else std::sort(order.begin(), order.end(), [](auto x, auto y) { return x->second.stamp < y->second.stamp; });
       for (auto it : order) {
-        if (cached_bytes <= peak_live) break;
+        if (cached_bytes <= keep) break;
         cudaFreeAsync(it->second.p, stream);
         held_bytes -= it->first;
         cached_bytes -= it->first;
