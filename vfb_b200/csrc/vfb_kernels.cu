@@ -52,8 +52,8 @@ __device__ __forceinline__ bool scan_compacts(const BatchDev& B) { return B.nins
 // of the table scan (256 threads, two words each) instead of by k_compact: a
 // kernel's start, ticket and look-back (4-5 us) cost more than the level's one
 // chunk.  One CTA would take the instances of a batch in turn: few only.
-__device__ __forceinline__ bool small_compact(const BatchDev& B, const InstDev& I) {
-  return scan_compacts(B) && I.plan_words <= kCompactWords;
+__device__ __forceinline__ bool small_compact(const BatchDev& B, uint64_t plan_words) {
+  return scan_compacts(B) && plan_words <= kCompactWords;
 }
 
 // ===================================================================== plan
@@ -682,7 +682,7 @@ __device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb, unsigned lon
 __global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev B) {
   step_entry();
   // the tuned CTA count of this step and its tiles (read together)
-  const unsigned long long cap = __ldcg(B.tickets + kTicketP1Blocks), total = __ldcg(B.p1_prefix + B.ninst);
+  const unsigned long long cap = ld_now(B.tickets[kTicketP1Blocks]), total = ld_now(B.p1_prefix[B.ninst]);
   const unsigned nb = cap && cap < gridDim.x ? (unsigned)cap : gridDim.x;
   if (blockIdx.x < nb) ph_p1(B, blockIdx.x, nb, total);
 }
@@ -711,31 +711,52 @@ __device__ __forceinline__ bool last_level(const InstDev& I) {
 }
 __device__ __forceinline__ bool last_unsolved(const InstDev& I) { return last_level(I) && I.best_cand == ~0ULL; }
 
-// What the scan of an instance's level visits: on the first attempt, when
-// every new slot is listed, the list; otherwise the whole table.
-struct ScanJob {
-  uint64_t entries, chunk;
-  bool listed;
+// What the table scan reads of an instance's record (all of it at once; the
+// scan itself changes none of it but the no_mask of a failed ownership check).
+struct ScanView {
+  unsigned long long k, best, newlist, tent, tmask;
+  uint64_t plan_words, entries, chunk;
+  const Slot* table;
+  const uint64_t* wins;
+  uint32_t* bitmap;
+  bool tail, runs, last, below, listed;
 };
-__device__ __forceinline__ ScanJob scan_job(const InstDev& I) {
-  ScanJob J;
-  J.listed = I.attempt == 1 && !I.no_list && I.n_newlist <= I.tent_cap;
-  J.entries = J.listed ? I.n_newlist : I.table_mask + 1;
-  J.chunk = I.scan_slots;
-  return J;
+__device__ __forceinline__ ScanView scan_view(const InstDev& I) {
+  const int status = ld_now(I.status), level = ld_now(I.level), max_size = ld_now(I.max_size),
+            attempt = ld_now(I.attempt), keep_last = ld_now(I.keep_last), otf = ld_now(I.on_the_fly),
+            no_mask = ld_now(I.no_mask), mask_off = ld_now(I.mask_off), tail = ld_now(I.p1_tail),
+            no_list = ld_now(I.no_list);
+  ScanView V;
+  V.best = ld_now(I.best_cand);
+  V.newlist = ld_now(I.n_newlist);
+  V.tent = ld_now(I.tent_cap);
+  V.tmask = ld_now(I.table_mask);
+  V.plan_words = ld_now(I.plan_words);
+  V.chunk = ld_now(I.scan_slots);
+  V.table = ld_now_ptr(I.table);
+  V.wins = ld_now_ptr(I.wins);
+  V.bitmap = ld_now_ptr(I.bitmap);
+  V.k = (unsigned long long)level;
+  V.tail = tail != 0;
+  V.runs = (status == ST_RUNNING) & (tail != 0) & (otf == 0);
+  V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0) & (no_mask == 0) & (mask_off == 0);
+  V.below = (V.best != ~0ULL) & (otf == 0) & (no_mask == 0) & (mask_off == 0);
+  // on the first attempt, when every new slot is listed, the list is visited;
+  // otherwise (a retried level) the whole table
+  V.listed = (attempt == 1) & (no_list == 0) & (V.newlist <= V.tent);
+  V.entries = V.listed ? V.newlist : V.tmask + 1;
+  return V;
 }
+__device__ __forceinline__ bool last_unsolved(const ScanView& V) { return V.last & (V.best == ~0ULL); }
 
 // Entries s0 .. s1-1 of the scan, by one CTA.
-__device__ void scan_chunk(InstDev& I, bool listed, uint64_t s0, uint64_t s1) {
+__device__ void scan_chunk(InstDev& I, const ScanView& V, uint64_t s0, uint64_t s1) {
   __shared__ unsigned long long s_w[32], s_b[32];
-  const unsigned long long k = (unsigned long long)I.level;
   // a level with a solution candidate (where it may skip operators) counts
-  // the owners below the candidate instead of marking owner bits: if the
-  // candidate owns its key (nearly always, and always with exact keys)
+  // the owners below the candidate instead of marking owner bits (V.below): if
+  // the candidate owns its key (nearly always, and always with exact keys)
   // that count is all the level needs; if not, the level is built again in
   // full (the ownership check below)
-  const unsigned long long bc = I.best_cand;
-  const bool below = below_mode(I);
   unsigned long long cnt = 0, nbelow = 0;
   // kScanBatch entries per thread at a time: their list reads, then their
   // payload reads, are in flight together
@@ -745,16 +766,16 @@ __device__ void scan_chunk(InstDev& I, bool listed, uint64_t s0, uint64_t s1) {
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
       const uint64_t e = e0 + (uint64_t)u * blockDim.x;
-      sl[u] = e < s1 ? (listed ? __ldcg(I.wins + e) : e) : ~0ULL;
+      sl[u] = e < s1 ? (V.listed ? __ldcg(V.wins + e) : e) : ~0ULL;
     }
 #pragma unroll
-    for (int u = 0; u < kScanBatch; ++u) pay[u] = sl[u] != ~0ULL ? __ldcg(&I.table[sl[u]].pay) : ~0ULL;
+    for (int u = 0; u < kScanBatch; ++u) pay[u] = sl[u] != ~0ULL ? __ldcg(&V.table[sl[u]].pay) : ~0ULL;
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
-      if ((pay[u] >> kPayShift) == k) {
+      if ((pay[u] >> kPayShift) == V.k) {
         const uint64_t g = pay[u] & kIdxMask;
-        if (below) nbelow += g < bc ? 1 : 0;
-        else atomicOr(I.bitmap + (g >> 5), 1u << (g & 31));
+        if (V.below) nbelow += g < V.best ? 1 : 0;
+        else atomicOr(V.bitmap + (g >> 5), 1u << (g & 31));
         ++cnt;
       }
     }
@@ -787,16 +808,16 @@ __device__ void ph_scan_tables(const BatchDev& B, unsigned bid, unsigned nb) {
   for (unsigned long long c = bid; c < total; c += nb) {
     const int b = find_owner(B.tscan_prefix, B.ninst, c);
     InstDev& I = B.inst[b];
-    if (COUNT_LAST && last_unsolved(I)) continue;
-    ScanJob J = scan_job(I);
-    if (J.listed) {
+    ScanView V = scan_view(I);
+    if (COUNT_LAST && last_unsolved(V)) continue;
+    if (V.listed) {
       // the list spread over the instance's chunks, at least a thread's entry each
-      const uint64_t nc = B.tscan_prefix[b + 1] - B.tscan_prefix[b], each = (J.entries + nc - 1) / nc;
-      if (each < J.chunk) J.chunk = (each + blockDim.x - 1) / blockDim.x * blockDim.x;
+      const uint64_t nc = B.tscan_prefix[b + 1] - B.tscan_prefix[b], each = (V.entries + nc - 1) / nc;
+      if (each < V.chunk) V.chunk = (each + blockDim.x - 1) / blockDim.x * blockDim.x;
     }
-    const uint64_t s0 = (c - B.tscan_prefix[b]) * J.chunk;
-    if (s0 >= J.entries) continue;   // (uniform over the CTA)
-    scan_chunk(I, J.listed, s0, s0 + J.chunk < J.entries ? s0 + J.chunk : J.entries);
+    const uint64_t s0 = (c - B.tscan_prefix[b]) * V.chunk;
+    if (s0 >= V.entries) continue;   // (uniform over the CTA)
+    scan_chunk(I, V, s0, s0 + V.chunk < V.entries ? s0 + V.chunk : V.entries);
   }
 }
 
@@ -847,30 +868,28 @@ __global__ void k_table_scan(const __grid_constant__ BatchDev B) {
   ph_table_scan(B, blockIdx.x, gridDim.x);
 }
 
-// A level's buffers against its nw owners: a shortfall asks the host for
-// memory before anything of the level is written (returns false).
-__device__ bool check_buffers(InstDev& I, unsigned long long nw, int sk) {
-  const unsigned long long fails = *(volatile unsigned long long*)&I.probe_fail;
-  const unsigned long long cap = I.table_mask + 1;
-  const int k = I.level;
-  int need = 0;
-  if (fails != 0 || 4 * (I.keys + nw) > 3 * cap) { need |= NEED_TABLE; I.need_amount[1] = 4 * (I.keys + nw) + 4096; }
-  if (nw > I.tent_cap) { need |= NEED_LIST; I.need_amount[2] = nw; }
-  if (!sk && I.lstart[k] + nw > I.row_cap) { need |= NEED_ROWS; I.need_amount[3] = I.lstart[k] + nw; }
-  if (!need) return true;
-  I.need = need;
-  I.planned = 0;
-  I.status = ST_NEED_MEM;
-  return false;
-}
-
-// An instance's part of the check: its row-emission items.
+// An instance's part of the check: its level's buffers against its owners (a
+// shortfall asks the host for memory before anything of the level is
+// written), its row-emission items.
 __device__ unsigned long long check_level(InstDev& I) {
-  if (*(volatile int*)&I.status != ST_RUNNING) return 0;
+  // (status, sol_known and n_wins may have been changed by this kernel: from the L2)
+  const int status = __ldcg(&I.status), sk = __ldcg(&I.sol_known), k = ld_now(I.level);
+  const unsigned long long wins = __ldcg(&I.n_wins), fresh = ld_now(I.n_new), fails = ld_now(I.probe_fail),
+                           keys = ld_now(I.keys), cap = ld_now(I.table_mask) + 1, tent = ld_now(I.tent_cap),
+                           row_cap = ld_now(I.row_cap), start = ld_now(I.lstart[k]);
   const bool counted = last_unsolved(I);
-  const unsigned long long nw = counted ? I.n_new : *(volatile unsigned long long*)&I.n_wins;
-  const int sk = *(volatile int*)&I.sol_known;
-  if (!check_buffers(I, nw, sk)) return 0;
+  if (status != ST_RUNNING) return 0;
+  const unsigned long long nw = counted ? fresh : wins;
+  int need = 0;
+  if (fails != 0 || 4 * (keys + nw) > 3 * cap) { need |= NEED_TABLE; I.need_amount[1] = 4 * (keys + nw) + 4096; }
+  if (nw > tent) { need |= NEED_LIST; I.need_amount[2] = nw; }
+  if (!sk && start + nw > row_cap) { need |= NEED_ROWS; I.need_amount[3] = start + nw; }
+  if (need) {
+    I.need = need;
+    I.planned = 0;
+    I.status = ST_NEED_MEM;
+    return 0;
+  }
   if (counted) I.n_wins = nw;
   if (counted || sk) return 0;
   int item = kEmitGroup;
@@ -882,19 +901,25 @@ __device__ unsigned long long check_level(InstDev& I) {
 // The check of few instances (see scan_compacts), by one CTA: their items'
 // prefix, and their small levels' owner bitmaps into the owner lists.  The
 // bitmap's words are read while thread 0 checks the buffers.
-__device__ void check_few(const BatchDev& B, unsigned long long* s_w) {
+__device__ void check_few(const BatchDev& B, const ScanView& solo, unsigned long long* s_w) {
   __shared__ int s_go;
   unsigned long long items = 0;
   for (int b = 0; b < B.ninst; ++b) {
     InstDev& I = B.inst[b];
-    const int st = *(volatile int*)&I.status;
-    const bool small = (st == ST_RUNNING || st == ST_NEED_MEM) && I.p1_tail && small_compact(B, I);
+    const ScanView V = B.ninst == 1 ? solo : scan_view(I);
+    const int st = __ldcg(&I.status);
+    const bool small = V.tail && small_compact(B, V.plan_words);
     uint32_t v[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const uint64_t w = 2 * threadIdx.x + j;
-      v[j] = small && w < I.plan_words ? __ldcg(I.bitmap + w) : 0u;
-      if (v[j]) I.bitmap[w] = 0u;
+      v[j] = small && w < V.plan_words ? __ldcg(V.bitmap + w) : 0u;
+    }
+    const bool has = (st == ST_RUNNING) | (st == ST_NEED_MEM);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (!has) v[j] = 0u;
+      if (v[j]) V.bitmap[2 * threadIdx.x + j] = 0u;
     }
     if (threadIdx.x == 0) {
       items += check_level(I);
@@ -903,10 +928,11 @@ __device__ void check_few(const BatchDev& B, unsigned long long* s_w) {
     }
     unsigned long long tot, pos = block_excl_scan(__popc(v[0]) + __popc(v[1]), s_w, tot);   // (barriers)
     if (s_go) {
+      uint64_t* wins = const_cast<uint64_t*>(V.wins);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         for (uint32_t bits = v[j]; bits; bits &= bits - 1)
-          I.wins[pos++] = (2 * threadIdx.x + j) * 32 + __ffs(bits) - 1;
+          wins[pos++] = (2 * threadIdx.x + j) * 32 + __ffs(bits) - 1;
       }
     }
     __syncthreads();
@@ -926,14 +952,20 @@ __global__ void __launch_bounds__(kScanThreadsCheck) k_table_scan_check(const __
   step_entry();
   const bool few = scan_compacts(B);
   unsigned long long part;
+  ScanView solo;   // the record of a single instance, read once
+  // chunks of the levels of few instances as they need them: a list of up to
+  // kListChunk slots takes one CTA
+  auto job = [&](const ScanView& V, uint64_t& chunk) -> uint64_t {
+    chunk = V.listed ? kListChunk : V.chunk;
+    return V.runs && !last_unsolved(V) ? V.entries : 0;
+  };
+  uint64_t chunk;
   if (few) {
-    // chunks as the levels need them: a list of up to kListChunk slots takes one CTA
     part = 1;
     for (int b = 0; b < B.ninst; ++b) {
-      const InstDev& I = B.inst[b];
-      if (I.status != ST_RUNNING || !I.p1_tail || I.on_the_fly || last_unsolved(I)) continue;
-      const ScanJob J = scan_job(I);
-      const uint64_t ch = J.listed ? kListChunk : J.chunk, nc = (J.entries + ch - 1) / ch;
+      const ScanView V = scan_view(B.inst[b]);
+      if (b == 0) solo = V;
+      const uint64_t n = job(V, chunk), nc = (n + chunk - 1) / chunk;
       part = nc > part ? nc : part;
     }
   } else {
@@ -944,14 +976,15 @@ __global__ void __launch_bounds__(kScanThreadsCheck) k_table_scan_check(const __
   }
   if (part > gridDim.x) part = gridDim.x;
   if (blockIdx.x >= part) return;
+  bool solved = !few;   // (few: some instance has a solution candidate)
   if (few) {
     for (int b = 0; b < B.ninst; ++b) {
       InstDev& I = B.inst[b];
-      if (I.status != ST_RUNNING || !I.p1_tail || I.on_the_fly || last_unsolved(I)) continue;
-      const ScanJob J = scan_job(I);
-      const uint64_t ch = J.listed ? kListChunk : J.chunk;
-      for (uint64_t s0 = blockIdx.x * ch; s0 < J.entries; s0 += part * ch)
-        scan_chunk(I, J.listed, s0, s0 + ch < J.entries ? s0 + ch : J.entries);
+      const ScanView V = B.ninst == 1 ? solo : scan_view(I);
+      solved |= V.best != ~0ULL;
+      const uint64_t n = job(V, chunk);
+      for (uint64_t s0 = blockIdx.x * chunk; s0 < n; s0 += part * chunk)
+        scan_chunk(I, V, s0, s0 + chunk < n ? s0 + chunk : n);
     }
   } else {
     ph_scan_tables<true>(B, blockIdx.x, (unsigned)part);
@@ -969,9 +1002,9 @@ __global__ void __launch_bounds__(kScanThreadsCheck) k_table_scan_check(const __
   if (few) {
     // (settled here, not before: every CTA derives part from the records, which
     // a failed ownership check changes)
-    ph_settle_solutions(B, 0, 1);
+    if (solved) ph_settle_solutions(B, 0, 1);
     __syncthreads();
-    check_few(B, s_w);
+    check_few(B, solo, s_w);
     return;
   }
   if (threadIdx.x == 0) s_carry = 0;
@@ -1276,8 +1309,9 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
     unsigned long long tiles = 0, chunks = 0, tchunks = 0;
     if (b < B.ninst) {
       InstDev& I = B.inst[b];
-      if (built && I.status == ST_RUNNING && I.planned == I.level) {
-        if (I.p1_tail) finish_one(I);
+      const int status = ld_now(I.status), planned = ld_now(I.planned), level = ld_now(I.level), tail = ld_now(I.p1_tail);
+      if (built && status == ST_RUNNING && planned == level) {
+        if (tail) finish_one(I);
         else I.p1_done += I.p1_step;   // a slice of the level's tiles ran
       }
       if (I.status == ST_RUNNING && I.planned != I.level) plan_one(I, scan_compacts(B));
@@ -1295,7 +1329,7 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
         const unsigned want = I.p1_blocks ? (unsigned)I.p1_blocks : ~0u;
         blocks = want > blocks ? want : blocks;
         if (I.p1_tail) {
-          chunks = last_level(I) || small_compact(B, I) ? 0 : (I.plan_words + kCompactWords - 1) / kCompactWords;
+          chunks = last_level(I) || small_compact(B, I.plan_words) ? 0 : (I.plan_words + kCompactWords - 1) / kCompactWords;
           tchunks = I.plan_tchunks;
         }
         run = 1;
@@ -1508,8 +1542,9 @@ __global__ void __launch_bounds__(kEmitThreads, 3) k_emit(const __grid_constant_
        item += nw) {
     const int b = find_owner(B.win_prefix, B.ninst, item);
     InstDev& I = B.inst[b];
-    if (I.status != ST_RUNNING) continue;
-    const int k = I.level, T = I.T, TP = I.TP;
+    const int status = ld_now(I.status), k = ld_now(I.level), T = ld_now(I.T), TP = ld_now(I.TP);
+    const uint64_t per = (uint64_t)ld_now(I.emit_item), nwin = ld_now(I.n_wins);
+    if (status != ST_RUNNING) continue;
     if (b != prev) {
       prev = b;
       __syncwarp();
@@ -1520,9 +1555,7 @@ __global__ void __launch_bounds__(kEmitThreads, 3) k_emit(const __grid_constant_
       }
       __syncwarp();
     }
-    const uint64_t per = (uint64_t)I.emit_item;
     const uint64_t o0 = (item - B.win_prefix[b]) * per;
-    const uint64_t nwin = I.n_wins;
     const int cnt = (int)(nwin - o0 < per ? nwin - o0 : per);
     const uint64_t r0 = I.lstart[k] + o0;
     // lane l decodes owner o0 + l
