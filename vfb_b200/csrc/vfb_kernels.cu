@@ -22,9 +22,9 @@
 //                 then the next level's candidate-block bases, P1 tiling and
 //                 buffer checks (LTL_BS.cu:1226-1488)
 //
-// The persistent, cluster and allocation-free solvers run the same phases
-// as k_plan, k_p1, k_table_scan, k_chunk_count/scan/emit, k_emit_rows,
-// k_finish.
+// The persistent and cluster solvers run the same phases (plan, P1, table
+// scan, chunk count/scan/emit, row emission, finish) inside one kernel, between
+// barriers.
 //
 // The reference's thrust::remove/copy_n compaction (storeUniqueLTLs
 // LTL_BS.cu:489-530) is replaced by the bitmap compaction; its racy
@@ -357,12 +357,6 @@ __device__ void ph_plan_prefix(const BatchDev& B) {
     B.tscan_prefix[b + 1] += B.tscan_prefix[b];
   }
   for (int i = 0; i < kTickets; ++i) B.tickets[i] = 0;
-}
-
-__global__ void __launch_bounds__(1024) k_plan(const __grid_constant__ BatchDev B) {
-  ph_plan(B, 0, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) ph_plan_prefix(B);
 }
 
 // ======================================================================= P1
@@ -864,10 +858,6 @@ __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
   ph_settle_solutions(B, bid, nb);
 }
 
-__global__ void k_table_scan(const __grid_constant__ BatchDev B) {
-  ph_table_scan(B, blockIdx.x, gridDim.x);
-}
-
 // An instance's part of the check: its level's buffers against its owners (a
 // shortfall asks the host for memory before anything of the level is
 // written), its row-emission items.
@@ -1048,10 +1038,6 @@ __device__ void ph_chunk_count(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_chunk_count(const __grid_constant__ BatchDev B) {
-  ph_chunk_count(B, blockIdx.x, gridDim.x);
-}
-
 // One CTA per instance: buffer checks for the level's new keys, scan of its
 // chunk counts.  The last CTA to finish (ticket) builds the owners' prefix
 // over instances.
@@ -1109,10 +1095,6 @@ __device__ void ph_chunk_scan(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void k_chunk_scan(const __grid_constant__ BatchDev B) {
-  ph_chunk_scan(B, blockIdx.x, gridDim.x);
-}
-
 // Emit set bits of each chunk in order; always clears the chunk's words.
 // The chunk is loaded coalesced into shared memory (padded rows), then every
 // thread scans its consecutive words.
@@ -1155,10 +1137,6 @@ __device__ void ph_chunk_emit(const BatchDev& B, unsigned bid, unsigned nb) {
   }
 }
 
-__global__ void __launch_bounds__(kChunkThreads) k_chunk_emit(const __grid_constant__ BatchDev B) {
-  ph_chunk_emit(B, blockIdx.x, gridDim.x);
-}
-
 // ================================================================ emit rows
 // Warp per winner, lane per trace word (coalesced row reads and writes).
 __device__ void ph_emit_rows(const BatchDev& B, unsigned bid, unsigned nb) {
@@ -1195,10 +1173,6 @@ __device__ void ph_emit_rows(const BatchDev& B, unsigned bid, unsigned nb) {
       record_unary(I, k, w, ((m >> 4) & 1u) | (m & 0xEu));   // (~ X F G)
     }
   }
-}
-
-__global__ void k_emit_rows(const __grid_constant__ BatchDev B) {
-  ph_emit_rows(B, blockIdx.x, gridDim.x);
 }
 
 // ================================================================== finish
@@ -1276,10 +1250,6 @@ __device__ void ph_finish(const BatchDev& B, unsigned bid, unsigned nb) {
     if (I.status == ST_RUNNING) finish_one(I);
     B.status_out[b] = make_int2(I.status, I.need);
   }
-}
-
-__global__ void k_finish(const __grid_constant__ BatchDev B) {
-  ph_finish(B, blockIdx.x, gridDim.x);
 }
 
 // ============================================================ level advance

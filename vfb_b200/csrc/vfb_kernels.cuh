@@ -5,8 +5,6 @@
 namespace vfb {
 
 constexpr int kChunkWords = 4096;     // bitmap words per compaction chunk (131072 bits)
-constexpr int kChunkThreads = 256;    // threads per compaction CTA
-constexpr int kScanThreads = 1024;
 constexpr int kScanSlots = 1024;      // hash-set slots per table-scan chunk (at least; more on
                                       // larger tables, see scan_slots)
 constexpr int kScanThreadsCheck = 256; // threads per k_table_scan_check CTA
@@ -43,10 +41,10 @@ struct BatchDev {
   unsigned long long* p1_prefix;        // [ninst+1] P1 tiles
   unsigned long long* chunk_prefix;     // [ninst+1] owner-bitmap chunks
   unsigned long long* tscan_prefix;     // [ninst+1] table-scan chunks
-  unsigned long long* win_prefix;       // [ninst+1] owners of new keys (k_emit_rows), or
+  unsigned long long* win_prefix;       // [ninst+1] owners of new keys (ph_emit_rows), or
                                         // row-emission groups (k_emit)
   unsigned int* chunk_cnt;              // [chunk_cap]
-  unsigned long long* chunk_base;       // [chunk_cap] chunk offsets (k_chunk_*), or the
+  unsigned long long* chunk_base;       // [chunk_cap] chunk offsets (ph_chunk_*), or the
                                         // look-back states of k_compact (flag << 62 | count)
   unsigned long long chunk_cap;
   unsigned long long* tickets;          // [kTickets]: P1 work ticket, scan done counter,
@@ -62,9 +60,9 @@ struct BatchDev {
 // Level step of the graph solver: k_p1, k_table_scan_check, k_compact,
 // k_emit, k_advance (k_advance also runs once, with built = 0, before the
 // first step of a launch).  k_table_scan_check adds the buffer checks to the
-// table scan; k_compact replaces k_chunk_count/scan/emit with one ordered
-// pass (decoupled look-back over the chunks); k_advance replaces k_finish +
-// k_plan + the loop control.  With loop != 0 it sets the graph's while
+// table scan; k_compact replaces the chunk count, scan and emission with one
+// ordered pass (decoupled look-back over the chunks); k_advance does the
+// finish, the plan and the loop control.  With loop != 0 it sets the graph's while
 // condition: some instance RUNNING, none waiting for memory, fewer than
 // max_iter steps.
 __global__ void k_advance(const __grid_constant__ BatchDev B, cudaGraphConditionalHandle handle, int built, int loop,
@@ -73,16 +71,7 @@ __global__ void k_table_scan_check(const __grid_constant__ BatchDev B);
 __global__ void k_compact(const __grid_constant__ BatchDev B);
 __global__ void k_emit(const __grid_constant__ BatchDev B);
 
-// Level-step kernels of the persistent, cluster and allocation-free solvers,
-// launched in this order for every level.
-__global__ void k_plan(const __grid_constant__ BatchDev B);
 __global__ void k_p1(const __grid_constant__ BatchDev B);
-__global__ void k_table_scan(const __grid_constant__ BatchDev B);
-__global__ void k_chunk_count(const __grid_constant__ BatchDev B);
-__global__ void k_chunk_scan(const __grid_constant__ BatchDev B);
-__global__ void k_chunk_emit(const __grid_constant__ BatchDev B);
-__global__ void k_emit_rows(const __grid_constant__ BatchDev B);
-__global__ void k_finish(const __grid_constant__ BatchDev B);
 
 // Persistent solver: the whole level loop in one cooperative launch (all CTAs
 // co-resident), the phases above separated by a bounded grid barrier.  Runs at

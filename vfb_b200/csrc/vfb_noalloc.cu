@@ -51,6 +51,14 @@ constexpr size_t kScratchBytes = 64ull << 20;   // VFB_NOALLOC_SCRATCH_BYTES in 
 constexpr uint64_t kNaSlots = 1ull << 19;        // hash-set slots (16 MiB)
 constexpr uint64_t kNaWords = 1ull << 20;        // candidate-bitmap words (32 Mi candidates)
 constexpr uint64_t kNaTents = 1ull << 19;        // owner-list entries
+// The look-back states of k_compact (a chunk of kCompactWords bitmap words each)
+// lie in the last entries of the owner list: a level has at most three quarters
+// of kNaSlots owners, so the list never reaches them.
+constexpr uint64_t kNaChunks = kNaWords / kCompactWords;
+static_assert(kNaTents - kNaChunks > kNaSlots / 4 * 3, "");
+// Levels launched per look at the status (a level that has nothing to do costs
+// five kernels of about 1.5 us, a look 10).
+constexpr int kNaLevels = 2;
 
 __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -136,7 +144,6 @@ struct Carver {
 // key layout of LTL_BS.cu:30-110).
 vfb_status fill_problem(const vfb_instance& in, InstDev& d) {
   std::memset(&d, 0, sizeof(d));
-  d.mask_off = 1;   // no level re-runs here: P1 never skips operators
   const int T = in.num_traces, A = in.num_vars;
   if (T < 1 || T > kMaxTraces || A < 1 || A > VFB_MAX_VARS || in.num_pos < 0 || in.num_pos > T)
     return VFB_LIMIT;
@@ -231,15 +238,16 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
   hB.tickets = cv.take<unsigned long long>(kTickets);
   hB.status_out = cv.take<int2>(1);
   hB.loop_iter = cv.take<unsigned long long>(1);
-  hB.chunk_cap = kNaWords / kChunkWords + 2;
-  hB.chunk_cnt = cv.take<unsigned int>(hB.chunk_cap);
-  hB.chunk_base = cv.take<unsigned long long>(hB.chunk_cap);
+  cv.take<unsigned int>(kNaWords / kChunkWords + 2);         // (unused, as above)
+  cv.take<unsigned long long>(kNaWords / kChunkWords + 2);
   d.table = cv.take<Slot>(kNaSlots);
   d.table_mask = kNaSlots - 1;
   d.bitmap = cv.take<uint32_t>(kNaWords);
   d.bitmap_words = kNaWords;
   d.wins = cv.take<uint64_t>(kNaTents);
-  d.tent_cap = kNaTents;
+  d.tent_cap = kNaTents - kNaChunks;
+  hB.chunk_cap = kNaChunks;
+  hB.chunk_base = reinterpret_cast<unsigned long long*>(d.wins + d.tent_cap);
   uint64_t* stage = cv.take<uint64_t>((size_t)d.T * d.A);   // the caller's words, as given
   const size_t used = ((cv.off + 255) & ~size_t(255)) + 512;   // + alignment of the last two carves
   const size_t per_row = (size_t)d.TP * 8 + 8;                  // row words + origin index
@@ -259,20 +267,20 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
   bool ok = cudaMemsetAsync(d.table, 0xFF, kNaSlots * sizeof(Slot), st) == cudaSuccess &&
             cudaMemsetAsync(d.bitmap, 0, kNaWords * 4, st) == cudaSuccess;
   // one copy of the words, turned into proposition rows on the device
-  ok = ok && cudaMemcpy(stage, inst->words, (size_t)d.T * d.A * 8, cudaMemcpyHostToDevice) == cudaSuccess;
+  ok = ok && cudaMemcpyAsync(stage, inst->words, (size_t)d.T * d.A * 8, cudaMemcpyHostToDevice, st) == cudaSuccess;
   h2d += (uint64_t)d.T * d.A * 8;
   if (ok) {
     k_na_rows<<<(d.A * d.TP + 255) / 256, 256, 0, st>>>(stage, d.T, d.A, d.TP, d.rows);
     ++launches;
     ok = cudaGetLastError() == cudaSuccess;
   }
-  ok = ok && cudaMemcpy(dI, &d, sizeof(InstDev), cudaMemcpyHostToDevice) == cudaSuccess;
+  ok = ok && cudaMemcpyAsync(dI, &d, sizeof(InstDev), cudaMemcpyHostToDevice, st) == cudaSuccess;
   h2d += sizeof(InstDev);
   if (!ok) return out->status = VFB_DEVICE_ERROR;
 
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int g = sms * 8, gc = sms * 2;
+  const int g = sms * 8;
   const int p1_smem = p1_smem_bytes(d.TP);
   int occ = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_p1, kTS, p1_smem);
@@ -281,21 +289,36 @@ extern "C" vfb_status vfb_solve_noalloc(const vfb_instance* inst, vfb_result* ou
   k_init<<<1, 256, 0, st>>>(hB);
   ++launches;
   int2 status{ST_RUNNING, 0};
-  for (int step = 0; step <= kMaxSize + 1; ++step) {
-    if (cudaMemcpy(&status, hB.status_out, sizeof(int2), cudaMemcpyDeviceToHost) != cudaSuccess)
+  const cudaGraphConditionalHandle none = 0;
+  k_advance<<<1, 32, 0, st>>>(hB, none, 0, 0, 0u);
+  ++launches;
+  // (a level is built twice at most: with relaxed keys its first solving
+  // candidate may share its key with an earlier one)
+  for (int step = 0; step <= 2 * kMaxSize + 2; ++step) {
+    for (int u = 0; u < kNaLevels; ++u) {
+      k_p1<<<p1_grid, kTS, p1_smem, st>>>(hB);
+      k_table_scan_check<<<g, kScanThreadsCheck, 0, st>>>(hB);
+      k_compact<<<g, kCompactThreads, 0, st>>>(hB);
+      k_emit<<<sms * 6, 256, 0, st>>>(hB);
+      k_advance<<<1, 32, 0, st>>>(hB, none, 1, 0, 0u);
+    }
+    launches += 5 * kNaLevels;
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpy(&status, hB.status_out, sizeof(int2), cudaMemcpyDeviceToHost) != cudaSuccess)
       return out->status = VFB_DEVICE_ERROR;
     d2h += sizeof(int2);
+    if (status.x == ST_NEED_MEM && status.y == 0) {
+      // nothing to grow: the level's first solution did not own its key while
+      // operators past it were skipped, and the level is built again in full
+      const int running = ST_RUNNING;
+      if (cudaMemcpyAsync(&dI->status, &running, sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        return out->status = VFB_DEVICE_ERROR;
+      k_advance<<<1, 32, 0, st>>>(hB, none, 0, 0, 0u);
+      ++launches;
+      h2d += sizeof(int);
+      continue;
+    }
     if (status.x != ST_RUNNING) break;
-    k_plan<<<1, 1024, 0, st>>>(hB);
-    k_p1<<<p1_grid, kTS, p1_smem, st>>>(hB);
-    k_table_scan<<<g, 256, 0, st>>>(hB);
-    k_chunk_count<<<gc, 256, 0, st>>>(hB);
-    k_chunk_scan<<<1, kScanThreads, 0, st>>>(hB);
-    k_chunk_emit<<<gc, kChunkThreads, 0, st>>>(hB);
-    k_emit_rows<<<g, 256, 0, st>>>(hB);
-    k_finish<<<1, 256, 0, st>>>(hB);
-    launches += 8;
-    if (cudaGetLastError() != cudaSuccess) return out->status = VFB_DEVICE_ERROR;
   }
   InstDev r;
   if (cudaMemcpy(&r, dI, sizeof(InstDev), cudaMemcpyDeviceToHost) != cudaSuccess)
