@@ -127,7 +127,6 @@ struct InstDev {
   uint64_t grp_base[kGroups][4];
   int p1_masked;   // a P1 tile of this attempt skipped operators past best_cand
   int no_mask;     // this level is re-run without skipping (set by the table scan)
-  int mask_off;    // never skip (contexts that cannot re-run a level)
   int rows_deferred;  // the projected rows of this level did not fit the budget: the level
                       // runs without them and the owner count after the table scan decides
   int ngroups;

@@ -73,7 +73,7 @@ __device__ void plan_one(InstDev& I, bool few) {
   const uint64_t keys = I.keys, table_cap = I.table_mask + 1, bitmap_words = I.bitmap_words,
                  row_cap = I.row_cap, tent_cap = I.tent_cap, promote_above = I.promote_above;
   const int attempt = I.attempt, attempt_level = I.attempt_level, rows_deferred = I.rows_deferred;
-  const int no_mask = (attempt_level == k) ? I.no_mask : 0, mask_off = I.mask_off;
+  const int no_mask = (attempt_level == k) ? I.no_mask : 0;
   // the first operand rows whose ~ X F G candidates satisfy the sample
   // (recorded when those rows were written)
   const int ulev[4] = {Ln, k - wX, k - wF, k - wG};
@@ -298,10 +298,9 @@ __device__ void plan_one(InstDev& I, bool few) {
     I.n_new = I.n_wins = I.probe_fail = I.n_newlist = 0;
     // A unary candidate recorded as satisfying the sample bounds the level's
     // first solution from the start, as if a P1 tile had found it: operators
-    // past it are skipped everywhere (not in a full re-run, nor where the
-    // level cannot be re-run)
+    // past it are skipped everywhere (not in a full re-run)
     uint64_t first = ~0ULL;
-    if (!no_mask && !mask_off) {
+    if (!no_mask) {
       const uint64_t ub[4] = {0, bx[0], bx[1], bx[2]};
 #pragma unroll
       for (int o = 0; o < 4; ++o) {
@@ -462,7 +461,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   const unsigned long long tmask = __ldcg(&Ip->table_mask), keys = __ldcg(&Ip->keys);
   const unsigned long long fails = __ldcg(&Ip->probe_fail), fresh = __ldcg(&Ip->n_new);
   const unsigned long long best = __ldcg(&Ip->best_cand);
-  const int may_skip = !__ldcg(&Ip->no_mask) && !__ldcg(&Ip->mask_off);
+  const int may_skip = !__ldcg(&Ip->no_mask);
   // lane l holds group boundaries 2l+1 and 2l+2; the group is the number of
   // boundaries at or below the tile (boundaries past the level's groups are
   // stale: read as never reached)
@@ -690,7 +689,7 @@ __global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev 
 // after P1 (the fields read are not written during the scan, except no_mask
 // by a failed ownership check, which rebuilds the level anyway).
 __device__ __forceinline__ bool below_mode(const InstDev& I) {
-  return I.best_cand != ~0ULL && !I.on_the_fly && !I.no_mask && !I.mask_off;
+  return I.best_cand != ~0ULL && !I.on_the_fly && !I.no_mask;
 }
 
 // Level max_size of a search (its first attempt): no later level reads its
@@ -701,7 +700,7 @@ __device__ __forceinline__ bool below_mode(const InstDev& I) {
 // in full.  (49 traces, size 9, nothing found: 8.7 M rows of the last level,
 // k_emit 3.2 -> 0.4 ms, the scan 0.45 -> 0.1, the solve 5.83 -> 2.9 ms.)
 __device__ __forceinline__ bool last_level(const InstDev& I) {
-  return I.level == I.max_size && I.attempt == 1 && !I.keep_last && !I.on_the_fly && !I.no_mask && !I.mask_off;
+  return I.level == I.max_size && I.attempt == 1 && !I.keep_last && !I.on_the_fly && !I.no_mask;
 }
 __device__ __forceinline__ bool last_unsolved(const InstDev& I) { return last_level(I) && I.best_cand == ~0ULL; }
 
@@ -718,7 +717,7 @@ struct ScanView {
 __device__ __forceinline__ ScanView scan_view(const InstDev& I) {
   const int status = ld_now(I.status), level = ld_now(I.level), max_size = ld_now(I.max_size),
             attempt = ld_now(I.attempt), keep_last = ld_now(I.keep_last), otf = ld_now(I.on_the_fly),
-            no_mask = ld_now(I.no_mask), mask_off = ld_now(I.mask_off), tail = ld_now(I.p1_tail),
+            no_mask = ld_now(I.no_mask), tail = ld_now(I.p1_tail),
             no_list = ld_now(I.no_list);
   ScanView V;
   V.best = ld_now(I.best_cand);
@@ -733,8 +732,8 @@ __device__ __forceinline__ ScanView scan_view(const InstDev& I) {
   V.k = (unsigned long long)level;
   V.tail = tail != 0;
   V.runs = (status == ST_RUNNING) & (tail != 0) & (otf == 0);
-  V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0) & (no_mask == 0) & (mask_off == 0);
-  V.below = (V.best != ~0ULL) & (otf == 0) & (no_mask == 0) & (mask_off == 0);
+  V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0) & (no_mask == 0);
+  V.below = (V.best != ~0ULL) & (otf == 0) & (no_mask == 0);
   // on the first attempt, when every new slot is listed, the list is visited;
   // otherwise (a retried level) the whole table
   V.listed = (attempt == 1) & (no_list == 0) & (V.newlist <= V.tent);
