@@ -23,6 +23,13 @@ constexpr int kTS = 128;              // stream rows per P1 tile (= threads per 
 constexpr int kTQ = 16;
 constexpr int kTQDefault = 16;        // staged rows per P1 tile unless the tune table says otherwise
 constexpr int kP1TileTarget = 4096;   // shrink the staged height until a level has this many tiles
+// Four lanes share a stream row (tiles of kTS/4 of them) at the levels of a few
+// instances, their keys not exact, that still have at most this many tiles
+// then: four CTAs on each of 148 SMs, so that the shorter tiles all run at once.
+// Rows over 64 words gain more from the shorter chain than eight such waves
+// cost (128 words: 614 us a solve with one wave, 604 with two, 588 with eight;
+// 19 words: 1478, 1482, 1500).
+constexpr int kP1SplitTiles = 592;
 // P1 launch shape per level band (tuned by the host): band b holds the levels
 // of 4^b to 4^(b+1)-1 candidates, the last band every larger level
 constexpr int kTuneBands = 16;
@@ -130,6 +137,7 @@ struct InstDev {
   int rows_deferred;  // the projected rows of this level did not fit the budget: the level
                       // runs without them and the owner count after the table scan decides
   int ngroups;
+  int p1_split;                // log2 of the lanes that share a stream row in P1 at this level (0, 2)
   int tq;                      // staged rows per P1 tile at this level (1..kTQ)
   int p1_blocks;               // P1 CTAs this level asks for (0: every resident CTA)
   unsigned long long promote_above;  // candidates per level above which the instance

@@ -72,6 +72,9 @@ __device__ void plan_one(InstDev& I, bool few) {
   const uint64_t lstart_prev = I.lstart[k - 1];
   const uint64_t keys = I.keys, table_cap = I.table_mask + 1, bitmap_words = I.bitmap_words,
                  row_cap = I.row_cap, tent_cap = I.tent_cap, promote_above = I.promote_above;
+  static_assert(kTS == 1 << 7, "");
+  const bool by_words = !exact_keys(I) && I.TP >= 8;   // (keys that take every word)
+  const uint64_t split_tiles = kP1SplitTiles * (I.TP > 64 ? 8 : 1);
   const int attempt = I.attempt, attempt_level = I.attempt_level, rows_deferred = I.rows_deferred;
   const int no_mask = (attempt_level == k) ? I.no_mask : 0;
   // the first operand rows whose ~ X F G candidates satisfy the sample
@@ -123,16 +126,18 @@ __device__ void plan_one(InstDev& I, bool few) {
   // launches fuse them.  The tiles of every staged height 2^0..2^5 are summed
   // on the way.
   int ng = 0;
-  uint64_t tl[6] = {0, 0, 0, 0, 0, 0};
+  uint64_t tl[6] = {0, 0, 0, 0, 0, 0}, tsplit = 0;   // (tsplit: kTS/4 rows a tile, one staged)
   auto add_tiles = [&](int kind, int la, int lb) {
     if (kind == 0) {
       const uint64_t st = (n[la] + kTS - 1) / kTS;
+      tsplit += (n[la] + kTS / 4 - 1) / (kTS / 4);
 #pragma unroll
       for (int u = 0; u < 6; ++u) tl[u] += (st + (1ULL << u) - 1) >> u;
     } else {
       const bool qleft = (la == lb) || (n[la] <= n[lb]);
       const uint64_t nS = qleft ? n[lb] : n[la], nQ = qleft ? n[la] : n[lb];
       const uint64_t st = (nS + kTS - 1) / kTS;
+      tsplit += (nS + kTS / 4 - 1) / (kTS / 4) * nQ;
 #pragma unroll
       for (int u = 0; u < 6; ++u) tl[u] += st * ((nQ + (1ULL << u) - 1) >> u);
     }
@@ -234,6 +239,12 @@ __device__ void plan_one(InstDev& I, bool few) {
   for (int u = 1; u < 6; ++u)
     if ((1 << u) <= rows_cap && tl[u] >= target) { lg = u; t = tl[u]; }
   I.tq = 1 << lg;
+  // four lanes to a stream row where the level then still runs in one wave
+  // (see kP1SplitTiles; in a batch the other instances fill the SMs)
+  const int split = few && by_words && !on_the_fly && lg == 0 && tsplit <= split_tiles ? 2 : 0;
+  const uint64_t height = kTS >> split;
+  if (split) t = tsplit;
+  I.p1_split = split;
   // group boundaries in tiles (ph_p1 reads the first ngroups of them)
   {
     uint64_t acc = 0;
@@ -243,11 +254,11 @@ __device__ void plan_one(InstDev& I, bool few) {
       const int la = weighted ? I.grp_la[q] : u_la(q);
       const int lb = weighted ? I.grp_lb[q] : u_lb(q);
       if (kind == 0) {
-        acc += ((n[la] + kTS - 1) / kTS + (1ULL << lg) - 1) >> lg;
+        acc += (((n[la] + height - 1) >> (7 - split)) + (1ULL << lg) - 1) >> lg;
       } else {
         const bool qleft = (la == lb) || (n[la] <= n[lb]);
         const uint64_t nS = qleft ? n[lb] : n[la], nQ = qleft ? n[la] : n[lb];
-        const uint64_t qt = (nQ + (1ULL << lg) - 1) >> lg, st = (nS + kTS - 1) / kTS;
+        const uint64_t qt = (nQ + (1ULL << lg) - 1) >> lg, st = (nS + height - 1) >> (7 - split);
         I.grp_qtiles[q] = (uint32_t)qt;
         acc += st * qt;
       }
@@ -414,7 +425,7 @@ __device__ __forceinline__ void p1_stage(const TileSh& P, QWord* sQ, QKey* sK) {
       if (c >= TP) c -= TP;
     }
   }
-  if (P.mode != KEY_HASH && !P.otf) {
+  if (P.mode != KEY_HASH && !P.otf && !P.split) {
     const int lane = threadIdx.x & 31;
     for (int r = threadIdx.x >> 5; r < P.nq; r += blockDim.x >> 5) {
       KeyAcc k;
@@ -456,6 +467,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   const int k = __ldcg(&Ip->level), T = __ldcg(&Ip->T), TP = __ldcg(&Ip->TP);
   const int stride = __ldcg(&Ip->stride1), mode = __ldcg(&Ip->key_mode), tq = __ldcg(&Ip->tq);
   const int lensum = __ldcg(&Ip->lensum), otf = __ldcg(&Ip->on_the_fly), nolist = __ldcg(&Ip->no_list);
+  const int split = __ldcg(&Ip->p1_split), height = kTS >> split;
   Slot* const table = (Slot*)__ldcg((const unsigned long long*)&Ip->table);
   const uint64_t* const rows = (const uint64_t*)__ldcg((const unsigned long long*)&Ip->rows);
   const unsigned long long tmask = __ldcg(&Ip->table_mask), keys = __ldcg(&Ip->keys);
@@ -492,6 +504,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   P.mode = mode;
   P.exact = mode == KEY_CONCAT && lensum <= 126;
   P.otf = otf;
+  P.split = split;
   P.nolist = nolist;
   P.tab = table;
   P.tmask = tmask;
@@ -504,7 +517,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   unsigned keep = 0xF;
   int all = gmask;
   if (kind == 0) {
-    const uint64_t s0 = within * tq * kTS, blocks = (ni - s0 + kTS - 1) / kTS;
+    const uint64_t s0 = within * tq * height, blocks = (ni - s0 + height - 1) >> (7 - split);
     P.nS = ni;
     P.s0 = s0;
     P.srows = rows + si * TP;
@@ -519,7 +532,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
     const uint64_t nS = qleft ? nj : ni, nQ = qleft ? ni : nj;
     uint64_t sq, qr;
     divmod64(within, qt, sq, qr);
-    const uint64_t s0 = sq * kTS, q0 = qr * tq;
+    const uint64_t s0 = sq * height, q0 = qr * tq;
     P.qleft = qleft;
     P.nS = nS;
     P.nQ = nQ;
@@ -582,19 +595,21 @@ __device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb, unsigned lon
     if (!idle && P.otf) {
       p1_solutions(P, rows, sQ, cnt);
     } else if (!idle) {
-      // a unary tile's rows, kTS a step, are one block of the level cache, read
+      // a unary tile's rows, kTS (>> split) a step, are one block of the level cache, read
       // once: the next step's are on their way to the L2 during this one
+      const int split = P.split;
+      const uint64_t height = kTS >> split;
       auto ahead = [&](uint64_t at) {
         if (threadIdx.x || at >= P.nS) return;
-        const uint64_t n = P.nS - at < (uint64_t)kTS ? P.nS - at : (uint64_t)kTS;
+        const uint64_t n = P.nS - at < height ? P.nS - at : height;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(rows + at * P.TP),
                      "r"((unsigned)(n * P.TP * 8)));
       };
       if (P.kind == 0 || P.q0 == 0) ahead(P.s0);
-      uint64_t a = P.s0 + threadIdx.x;
+      uint64_t a = P.s0 + (threadIdx.x >> split);
       const uint64_t* row = rows + (a < P.nS ? a : P.nS - 1) * P.TP;
       KeyAcc sk{0, 0};
-      if (P.kind && P.mode != KEY_HASH)
+      if (P.kind && P.mode != KEY_HASH && !split)
         sk = P.mode == KEY_SAMPLED ? row_bits<KEY_SAMPLED>(P, row) : row_bits<KEY_CONCAT>(P, row);
       const bool one = P.mask == 1;
       for (int q = 0; q < P.nq;) {
@@ -602,22 +617,28 @@ __device__ void ph_p1(const BatchDev& B, unsigned bid, unsigned nb, unsigned lon
         Cands C;
         C.ok = 0;
         if (P.kind == 0) {
-          a = P.s0 + (uint64_t)q * kTS + threadIdx.x;
+          a = P.s0 + (uint64_t)q * height + (threadIdx.x >> split);
           row = rows + (a < P.nS ? a : P.nS - 1) * P.TP;
-          if (q + 1 < P.nq) ahead(P.s0 + (uint64_t)(q + 1) * kTS);
-          switch (P.mode) {
+          if (q + 1 < P.nq) ahead(P.s0 + (uint64_t)(q + 1) * height);
+          if (!split) switch (P.mode) {
             case KEY_HASH: one ? p1_unary<KEY_HASH, 1>(P, row, a, C, cnt) : p1_unary<KEY_HASH, 4>(P, row, a, C, cnt); break;
             case KEY_SAMPLED:
               one ? p1_unary<KEY_SAMPLED, 1>(P, row, a, C, cnt) : p1_unary<KEY_SAMPLED, 4>(P, row, a, C, cnt);
               break;
             default: one ? p1_unary<KEY_CONCAT, 1>(P, row, a, C, cnt) : p1_unary<KEY_CONCAT, 4>(P, row, a, C, cnt);
           }
-        } else {
+          else if (P.mode == KEY_HASH) p1_unary_split<KEY_HASH>(P, row, a, C, cnt);
+          else p1_unary_split<KEY_CONCAT>(P, row, a, C, cnt);
+        } else if (!split) {
           switch (P.mode) {
             case KEY_HASH: done = p1_pair<KEY_HASH>(P, row, sk, sQ, sK, q, C, cnt); break;
             case KEY_SAMPLED: done = p1_pair<KEY_SAMPLED>(P, row, sk, sQ, sK, q, C, cnt); break;
             default: done = p1_pair<KEY_CONCAT>(P, row, sk, sQ, sK, q, C, cnt);
           }
+        } else {
+          const QWord* qw = sQ + q * P.TP;
+          if (P.mode == KEY_HASH) p1_pair_split<KEY_HASH>(P, row, qw, P.q0 + q, a, C, cnt);
+          else p1_pair_split<KEY_CONCAT>(P, row, qw, P.q0 + q, a, C, cnt);
         }
         q += done;
         // two candidates at a time, so that the queue stays short (the drain's

@@ -383,8 +383,9 @@ struct TileSh {
   int otf;          // on-the-fly level: solution test only, nothing inserted
   int nolist;       // new slots are not listed (the table scan reads the whole table)
   int exact;        // every bit of every trace is in the key (KEY_CONCAT, no field cut)
+  int split;        // log2 of the lanes that share a stream row
   uint64_t s0, q0, nS, nQ;
-  int nq;           // staged rows of this tile, or blocks of kTS stream rows of a unary one
+  int nq;           // staged rows of this tile, or blocks of kTS (>> split) stream rows of a unary one
   const uint64_t *srows, *qrows;   // the stream operand's level; this tile's staged rows
   Slot* tab;
   uint64_t tmask;
@@ -930,6 +931,107 @@ __device__ __forceinline__ void p1_pair_bits(const TileSh& P, const uint64_t* sr
     for (int u = 0; u < N; ++u) key_final<MODE>(k[u], C.h[u], C.l[u]);
   }
   take_pair<KEYS>(P, q, s, 0, bad, C, cnt);
+}
+
+// ---- four lanes to a stream row (small levels, keys that need the words)
+// A level that does not fill the SMs is bound by one thread's chain over the
+// words of its row: a load's latency every four words and some sixty dependent
+// instructions a word.  Here lane s of four takes the words 8i + 2s and the
+// next one.  Keys are XOR folds (hashes, or bit fields side by side) and the
+// step-0 tests ORs, so the lanes' parts
+// combine in two exchanges, which leave candidate s in lane s: one key to
+// finish and to queue per lane.  128 traces with sampled keys, levels up to
+// 72,000 candidates: the solve 778 -> 603 us; 40 traces, hash keys: k_p1 of
+// five levels 92 -> 70 us.  Copies for fewer operators, or per bit-field rule,
+// only added code: a small level runs its instructions from a cold cache.
+// MODE: KEY_HASH, or KEY_CONCAT for either bit-field key.
+// ops(t, w, c): the four candidates' words from word t of the row.
+template <int MODE, typename F>
+__device__ __forceinline__ void fold_split(const TileSh& P, const uint64_t* row, F&& ops, Cands& C, uint32_t& bad) {
+  const int sub = threadIdx.x & 3, TP = P.TP, half = P.half;
+  KeyAcc k[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) k[j] = KeyAcc{0, 0};
+  uint32_t miss = 0;
+  int t = 2 * sub;
+  uint64_t v[2] = {0, 0};
+  if (t < TP) ld_row2(row + t, v[0], v[1]);
+#pragma unroll 1
+  for (; t < TP; t += 8) {
+    uint64_t n[2];
+    ld_row2(row + (t + 8 < TP ? t + 8 : t), n[0], n[1]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint64_t c[4];
+      ops(t + u, v[0], c);
+      v[0] = v[1];
+      const uint32_t lab = P.tr[t + u].lab;
+      const uint64_t below = t + u < half ? ~0ULL : 0ULL;   // (the words below T/2 fold into h)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        miss |= ((lo32(c[j]) ^ lab) & 1u) << j;
+        if constexpr (MODE == KEY_HASH) {
+          const uint64_t x = splitmix_mul(c[j] ^ (c[j] >> 30));
+          k[j].a0 ^= x & ~below;
+          k[j].a1 ^= x & below;
+        } else {
+          const int at = P.off[t + u], wd = P.wid[t + u], L = P.len[t + u];
+          if (P.mode == KEY_SAMPLED) key_word<KEY_SAMPLED>(k[j], c[j], t + u, 0, at, wd, P.stride, L);
+          else key_word<KEY_CONCAT>(k[j], c[j], t + u, 0, at, wd, P.stride, L);
+        }
+      }
+    }
+    v[0] = n[0];
+    v[1] = n[1];
+  }
+  // lanes 0, 1 of four keep candidates 0, 1 and get the others' part of them
+  // (2, 3 likewise), then each lane its own
+  const unsigned full = 0xffffffffu;
+  const bool b2 = sub & 2, b1 = sub & 1;
+  auto give = [&](bool up, KeyAcc& x, const KeyAcc& y, int o) {   // x: the kept one of the two
+    const uint64_t a0 = __shfl_xor_sync(full, up ? x.a0 : y.a0, o), a1 = __shfl_xor_sync(full, up ? x.a1 : y.a1, o);
+    x = KeyAcc{(up ? y.a0 : x.a0) ^ a0, (up ? y.a1 : x.a1) ^ a1};
+  };
+  give(b2, k[0], k[2], 2);
+  give(b2, k[1], k[3], 2);
+  give(b1, k[0], k[1], 1);
+  key_final<MODE>(k[0], C.h[0], C.l[0]);
+  miss |= __shfl_xor_sync(full, miss, 1);
+  miss |= __shfl_xor_sync(full, miss, 2);
+  bad = miss >> sub;
+}
+
+// ~ X F G of row a (one variant: a small level's masked operators cost less
+// than another copy of the code).
+template <int MODE>
+__device__ __forceinline__ void p1_unary_split(const TileSh& P, const uint64_t* row, uint64_t a, Cands& C, P1Count& cnt) {
+  uint32_t bad;
+  fold_split<MODE>(P, row, [&](int t, uint64_t w, uint64_t (&c)[4]) {
+    c[0] = ~w & P.tr[t].lm;
+    c[1] = w >> 1;
+    c[2] = w_fin(w);
+    c[3] = w & ~w_fin(c[0]);
+  }, C, bad);
+  const int o = threadIdx.x & 3;
+  take_cand(C, 0, a < P.nS && ((P.mask >> o) & 1), P.gb[o] + a, bad, cnt);
+}
+
+// & | qUs sUq of staged row q (words qw) and stream row s.
+template <int MODE>
+__device__ __forceinline__ void p1_pair_split(const TileSh& P, const uint64_t* row, const QWord* qw, uint64_t q, uint64_t s,
+                                              Cands& C, P1Count& cnt) {
+  uint32_t bad;
+  fold_split<MODE>(P, row, [&](int t, uint64_t w, uint64_t (&c)[4]) {
+    const QWord x = qw[t];
+    const uint64_t rev = __brevll(w);
+    c[0] = w & x.w;
+    c[1] = w | x.w;
+    c[2] = __brevll(until_rev(x.rev, rev));
+    c[3] = __brevll(until_rev(rev, x.rev));
+  }, C, bad);
+  const int o = threadIdx.x & 3;
+  const uint64_t qs = q * P.nS + s, sq = s * P.nQ + q;
+  take_cand(C, 0, s < P.nS && ((P.mask >> o) & 1), P.gb[o] + (o == 2 || (o < 2 && P.qleft) ? qs : sq), bad, cnt);
 }
 
 // Staged row q of a binary tile (and the next, where two are taken at a time)
