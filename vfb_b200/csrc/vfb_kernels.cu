@@ -1285,15 +1285,23 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
   __shared__ unsigned long long s_w3[32][3];
   __shared__ unsigned long long s_carry[3];
   step_entry();
-  if (threadIdx.x == 0) {
-    s_run = 0;
-    s_need = 0;
-    s_blocks = 0;
-    s_carry[0] = s_carry[1] = s_carry[2] = 0;
+  // A few instances are warp 0's lanes: their prefixes and totals take a few
+  // shuffles instead of block scans and barriers (the kernel runs its code once,
+  // from a cold instruction cache): an eight-level search 677 -> 670 us.
+  const bool few = scan_compacts(B);
+  if (few && threadIdx.x >= 32) return;
+  if (!few) {
+    if (threadIdx.x == 0) {
+      s_run = 0;
+      s_need = 0;
+      s_blocks = 0;
+      s_carry[0] = s_carry[1] = s_carry[2] = 0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
   int run = 0, need = 0;
   unsigned blocks = 0;   // CTAs the step's P1 asks for (~0u: every resident CTA)
+  unsigned long long nchunks = 0;
   for (int base = 0; base < B.ninst; base += blockDim.x) {
     const int b = base + threadIdx.x;
     unsigned long long tiles = 0, chunks = 0, tchunks = 0;
@@ -1304,7 +1312,7 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
         if (tail) finish_one(I);
         else I.p1_done += I.p1_step;   // a slice of the level's tiles ran
       }
-      if (I.status == ST_RUNNING && I.planned != I.level) plan_one(I, scan_compacts(B));
+      if (I.status == ST_RUNNING && I.planned != I.level) plan_one(I, few);
       if (I.status == ST_RUNNING) {
         // this step's slice of P1 tiles: all that remain, or the quota's worth
         const unsigned long long left = I.plan_tiles - I.p1_done;
@@ -1327,6 +1335,23 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
       need |= (I.status == ST_NEED_MEM);
       B.status_out[b] = make_int2(I.status, I.need);
     }
+    if (few) {
+      unsigned long long x[3] = {tiles, chunks, tchunks};
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const unsigned long long y = __shfl_up_sync(0xffffffffu, x[c], o);
+          if ((int)threadIdx.x >= o) x[c] += y;
+        }
+      if (b < B.ninst) {
+        B.p1_prefix[b + 1] = x[0];
+        B.chunk_prefix[b + 1] = x[1];
+        B.tscan_prefix[b + 1] = x[2];
+      }
+      nchunks = __shfl_sync(0xffffffffu, x[1], 3);
+      break;
+    }
     // inclusive prefixes over this block of instances, carried across blocks
     const unsigned long long v[3] = {tiles, chunks, tchunks};
     unsigned long long ex[3], tot[3];
@@ -1344,24 +1369,33 @@ __global__ void __launch_bounds__(kAdvanceThreads) k_advance(const __grid_consta
     }
     __syncthreads();
   }
-  if (run) atomicOr(&s_run, 1);
-  if (need) atomicOr(&s_need, 1);
-  if (blocks) atomicMax(&s_blocks, blocks);
-  __syncthreads();
+  if (few) {
+    run = __any_sync(0xffffffffu, run);
+    need = __any_sync(0xffffffffu, need);
+    blocks = __reduce_max_sync(0xffffffffu, blocks);
+  } else {
+    if (run) atomicOr(&s_run, 1);
+    if (need) atomicOr(&s_need, 1);
+    if (blocks) atomicMax(&s_blocks, blocks);
+    __syncthreads();
+    run = s_run;
+    need = s_need;
+    blocks = s_blocks;
+    nchunks = s_carry[1];
+  }
   if (threadIdx.x == 0) {
     B.p1_prefix[0] = 0;
     B.chunk_prefix[0] = 0;
     B.tscan_prefix[0] = 0;
     for (int i = 0; i < 4; ++i) B.tickets[i] = 0;
-    B.tickets[kTicketP1Blocks] = s_blocks == ~0u ? 0 : s_blocks;
+    B.tickets[kTicketP1Blocks] = blocks == ~0u ? 0 : blocks;
   }
-  __syncthreads();
-  const unsigned long long nchunks = s_carry[1];
-  for (unsigned long long c = threadIdx.x; c < nchunks; c += blockDim.x) B.chunk_base[c] = 0;
+  const unsigned stride = few ? 32u : blockDim.x;
+  for (unsigned long long c = threadIdx.x; c < nchunks; c += stride) B.chunk_base[c] = 0;
   if (loop && threadIdx.x == 0) {
     // (the launch's leading advance starts the count)
     const unsigned long long it = *B.loop_iter = built ? *B.loop_iter + 1 : 1;
-    const bool more = s_run && !s_need && it < max_iter;
+    const bool more = run && !need && it < max_iter;
     cudaGraphSetConditional(handle, more ? 1u : 0u);
   }
 }
