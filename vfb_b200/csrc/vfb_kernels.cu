@@ -707,10 +707,14 @@ __global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev 
 // payload (~0) carries no level <= 32.  One warp per instance also settles
 // whether the recorded solution candidate owns its key.
 // The table scan's counting mode at a level that has a solution candidate
-// after P1 (the fields read are not written during the scan, except no_mask
-// by a failed ownership check, which rebuilds the level anyway).
+// after P1.  The fields read are not written during the scan, except no_mask:
+// a failed ownership check sets it while other CTAs of a batch still scan the
+// instance's chunks.  A first attempt therefore goes by attempt alone (its
+// no_mask was 0 when it was planned): it must not change to marking owners
+// half-way, since a last level has no compaction to clear the bitmap
+// (last_level).  A later attempt may: its bitmap is always compacted.
 __device__ __forceinline__ bool below_mode(const InstDev& I) {
-  return I.best_cand != ~0ULL && !I.on_the_fly && !I.no_mask;
+  return I.best_cand != ~0ULL && !I.on_the_fly && (I.attempt == 1 || !I.no_mask);
 }
 
 // Level max_size of a search (its first attempt): no later level reads its
@@ -721,12 +725,13 @@ __device__ __forceinline__ bool below_mode(const InstDev& I) {
 // in full.  (49 traces, size 9, nothing found: 8.7 M rows of the last level,
 // k_emit 3.2 -> 0.4 ms, the scan 0.45 -> 0.1, the solve 5.83 -> 2.9 ms.)
 __device__ __forceinline__ bool last_level(const InstDev& I) {
-  return I.level == I.max_size && I.attempt == 1 && !I.keep_last && !I.on_the_fly && !I.no_mask;
+  return I.level == I.max_size && I.attempt == 1 && !I.keep_last && !I.on_the_fly;
 }
 __device__ __forceinline__ bool last_unsolved(const InstDev& I) { return last_level(I) && I.best_cand == ~0ULL; }
 
 // What the table scan reads of an instance's record (all of it at once; the
-// scan itself changes none of it but the no_mask of a failed ownership check).
+// scan itself changes none of it but the no_mask of a failed ownership check,
+// see below_mode).
 struct ScanView {
   unsigned long long k, best, newlist, tent, tmask;
   uint64_t plan_words, entries, chunk;
@@ -753,8 +758,8 @@ __device__ __forceinline__ ScanView scan_view(const InstDev& I) {
   V.k = (unsigned long long)level;
   V.tail = tail != 0;
   V.runs = (status == ST_RUNNING) & (tail != 0) & (otf == 0);
-  V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0) & (no_mask == 0);
-  V.below = (V.best != ~0ULL) & (otf == 0) & (no_mask == 0);
+  V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0);
+  V.below = (V.best != ~0ULL) & (otf == 0) & ((attempt == 1) | (no_mask == 0));
   // on the first attempt, when every new slot is listed, the list is visited;
   // otherwise (a retried level) the whole table
   V.listed = (attempt == 1) & (no_list == 0) & (V.newlist <= V.tent);
