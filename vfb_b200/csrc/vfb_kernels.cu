@@ -738,7 +738,7 @@ struct ScanView {
   const Slot* table;
   const uint64_t* wins;
   uint32_t* bitmap;
-  bool tail, runs, last, below, listed;
+  bool live, tail, runs, last, below, listed;   // live: its buffers are held
 };
 __device__ __forceinline__ ScanView scan_view(const InstDev& I) {
   const int status = ld_now(I.status), level = ld_now(I.level), max_size = ld_now(I.max_size),
@@ -756,6 +756,7 @@ __device__ __forceinline__ ScanView scan_view(const InstDev& I) {
   V.wins = ld_now_ptr(I.wins);
   V.bitmap = ld_now_ptr(I.bitmap);
   V.k = (unsigned long long)level;
+  V.live = (status == ST_RUNNING) | (status == ST_NEED_MEM);
   V.tail = tail != 0;
   V.runs = (status == ST_RUNNING) & (tail != 0) & (otf == 0);
   V.last = (level == max_size) & (attempt == 1) & (keep_last == 0) & (otf == 0);
@@ -915,27 +916,25 @@ __device__ unsigned long long check_level(InstDev& I) {
 
 // The check of few instances (see scan_compacts), by one CTA: their items'
 // prefix, and their small levels' owner bitmaps into the owner lists.  The
-// bitmap's words are read while thread 0 checks the buffers.
+// bitmap's words are read while thread 0 checks the buffers.  The record of an
+// instance that is done, refused or gave way still names buffers that may be
+// somebody else's, or unmapped, by now: nothing behind it is read.
 __device__ void check_few(const BatchDev& B, const ScanView& solo, unsigned long long* s_w) {
   __shared__ int s_go;
   unsigned long long items = 0;
   for (int b = 0; b < B.ninst; ++b) {
     InstDev& I = B.inst[b];
     const ScanView V = B.ninst == 1 ? solo : scan_view(I);
-    const int st = __ldcg(&I.status);
-    const bool small = V.tail && small_compact(B, V.plan_words);
+    const bool small = V.live && V.tail && small_compact(B, V.plan_words);
     uint32_t v[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const uint64_t w = 2 * threadIdx.x + j;
       v[j] = small && w < V.plan_words ? __ldcg(V.bitmap + w) : 0u;
     }
-    const bool has = (st == ST_RUNNING) | (st == ST_NEED_MEM);
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      if (!has) v[j] = 0u;
+    for (int j = 0; j < 2; ++j)
       if (v[j]) V.bitmap[2 * threadIdx.x + j] = 0u;
-    }
     if (threadIdx.x == 0) {
       items += check_level(I);
       B.win_prefix[b + 1] = items;
