@@ -886,14 +886,16 @@ __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
 
 // An instance's part of the check: its level's buffers against its owners (a
 // shortfall asks the host for memory before anything of the level is
-// written), its row-emission items.
+// written), its row-emission items.  The owners are known after the level's
+// last slice of P1 tiles; an earlier slice (n_wins still 0) only stops at a
+// failed probe.
 __device__ unsigned long long check_level(InstDev& I) {
   // (status, sol_known and n_wins may have been changed by this kernel: from the L2)
   const int status = __ldcg(&I.status), sk = __ldcg(&I.sol_known), k = ld_now(I.level);
   const unsigned long long wins = __ldcg(&I.n_wins), fresh = ld_now(I.n_new), fails = ld_now(I.probe_fail),
                            keys = ld_now(I.keys), cap = ld_now(I.table_mask) + 1, tent = ld_now(I.tent_cap),
                            row_cap = ld_now(I.row_cap), start = ld_now(I.lstart[k]);
-  const bool counted = last_unsolved(I);
+  const bool counted = ld_now(I.p1_tail) != 0 && last_unsolved(I);
   if (status != ST_RUNNING) return 0;
   const unsigned long long nw = counted ? fresh : wins;
   int need = 0;
