@@ -81,9 +81,23 @@ __host__ __device__ inline int tune_band(unsigned long long cands) {
 
 // Per-instance device state.  Kernels read everything they need from here,
 // so one captured launch sequence serves every level and every batch.
+// Whether every word's bits lie within its trace.  The operators work on whole
+// words, and a bit past the trace reaches into it through F, G and U: the keys
+// hold all there is to a set only without such bits.
+inline bool words_within(const uint64_t* words, const int* lengths, int T, int A) {
+  for (int i = 0; i < T; ++i) {
+    if (lengths[i] >= 64) continue;
+    for (int v = 0; v < A; ++v)
+      if (words[(size_t)i * A + v] >> lengths[i]) return false;
+  }
+  return true;
+}
+
 struct InstDev {
   // ---- problem (written once by the host)
-  int T, TP, A, npos, max_size, key_mode, stride1, lensum;
+  int T, TP, A, npos, max_size, key_mode, stride1;
+  int exact;                   // the key holds every bit of every word: KEY_CONCAT, no field cut, and
+                               // no proposition has a bit past its trace (words_within)
   uint8_t len[kMaxTraces];
   uint8_t off[kMaxTraces];     // bit offset of the trace's key field (<=126)
   uint8_t width[kMaxTraces];   // key field width (0 when past bit 126)

@@ -1081,7 +1081,7 @@ struct Engine {
     }
     d.npos = in.num_pos;
     d.max_size = in.max_size;
-    d.lensum = S;
+    d.exact = S <= 126 && words_within(in.words, in.lengths, T, A);
     d.stride1 = 1;
     for (int i = 0; i < T; ++i) {
       d.len[i] = (uint8_t)in.lengths[i];

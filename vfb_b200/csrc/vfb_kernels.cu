@@ -466,7 +466,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   }
   const int k = __ldcg(&Ip->level), T = __ldcg(&Ip->T), TP = __ldcg(&Ip->TP);
   const int stride = __ldcg(&Ip->stride1), mode = __ldcg(&Ip->key_mode), tq = __ldcg(&Ip->tq);
-  const int lensum = __ldcg(&Ip->lensum), otf = __ldcg(&Ip->on_the_fly), nolist = __ldcg(&Ip->no_list);
+  const int exact = __ldcg(&Ip->exact), otf = __ldcg(&Ip->on_the_fly), nolist = __ldcg(&Ip->no_list);
   const int split = __ldcg(&Ip->p1_split), height = kTS >> split;
   Slot* const table = (Slot*)__ldcg((const unsigned long long*)&Ip->table);
   const uint64_t* const rows = (const uint64_t*)__ldcg((const unsigned long long*)&Ip->rows);
@@ -502,7 +502,7 @@ __device__ __forceinline__ void p1_setup(InstDev* Ip, int b, uint64_t local, Til
   P.half = T / 2;
   P.stride = stride;
   P.mode = mode;
-  P.exact = mode == KEY_CONCAT && lensum <= 126;
+  P.exact = exact;
   P.otf = otf;
   P.split = split;
   P.nolist = nolist;
@@ -1550,13 +1550,12 @@ __device__ __forceinline__ ulonglong2 emit_words(int op, ulonglong2 l, ulonglong
   }
 }
 
-// emit_miss of two words (see there; a word covers its whole trace when it
-// equals the length mask).
+// emit_miss of two words (see there).
 __device__ __forceinline__ unsigned emit_test(uint64_t w0, uint64_t w1, ulonglong2 lm, uint2 lab) {
   const unsigned x0 = (unsigned)w0 ^ lab.x, x1 = (unsigned)w1 ^ lab.y;
   const bool l0 = lab.x != 0, l1 = lab.y != 0;
   const bool f = ((w0 != 0) != l0) || ((w1 != 0) != l1);
-  const bool g = ((w0 == lm.x) != l0) || ((w1 == lm.y) != l1);
+  const bool g = (((~w0 & lm.x) == 0) != l0) || (((~w1 & lm.y) == 0) != l1);
   return ((x0 | x1) & 3u) | (f ? 4u : 0u) | (g ? 8u : 0u) | ((~(x0 & x1) & 1u) << 4);
 }
 

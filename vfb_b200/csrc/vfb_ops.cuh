@@ -370,7 +370,7 @@ __device__ inline void cand_key(const InstDev& I, const Cand& c, uint64_t& h, ui
 // ======================================================================= P1
 // Shared per-tile parameters.  s: the stream operand (a row per thread), q:
 // the staged operand (up to kTQ rows, read by every thread).
-__device__ __forceinline__ bool exact_keys(const InstDev& I) { return I.key_mode == KEY_CONCAT && I.lensum <= 126; }
+__device__ __forceinline__ bool exact_keys(const InstDev& I) { return I.exact != 0; }
 
 struct __align__(16) TraceSh {
   uint64_t lm;     // length mask
@@ -382,7 +382,7 @@ struct TileSh {
                     // operators it evaluates
   int otf;          // on-the-fly level: solution test only, nothing inserted
   int nolist;       // new slots are not listed (the table scan reads the whole table)
-  int exact;        // every bit of every trace is in the key (KEY_CONCAT, no field cut)
+  int exact;        // every bit of every word is in the key (see InstDev::exact)
   int split;        // log2 of the lanes that share a stream row
   uint64_t s0, q0, nS, nQ;
   int nq;           // staged rows of this tile, or blocks of kTS (>> split) stream rows of a unary one
