@@ -301,13 +301,23 @@ struct Engine {
       return p;
     }
     // a large fresh block is rounded up (by an eighth at most) while little of
-    // the budget is in use: the next solve, whose needs differ by a percent,
-    // then reuses it instead of mapping memory (10 ms per GB)
-    if (bytes >= ((size_t)16 << 20)) {
+    // the budget and of the device's free memory is in use: the next solve,
+    // whose needs differ by a percent, then reuses it instead of mapping memory
+    // (10 ms per GB).  Its capacity is what was asked for, so that buffer sizes,
+    // and what fits a request's byte cap, do not depend on the rounding, and
+    // what it takes from later growth is under a percent of either.  (With a
+    // third of the budget as the bound and rounded capacities, a search that
+    // needs 5.5 GB failed beside another user of the GPU up to 6.0 GB free.)
+    // Not in a serving session, whose arena holds its memory.
+    const size_t asked = bytes;
+    if (!single_step && bytes >= ((size_t)16 << 20)) {
       size_t unit = (size_t)1 << 20;
       while (unit * 16 <= bytes) unit *= 2;
-      const size_t up = (bytes + unit - 1) / unit * unit;
-      if (!mem_limit || held_bytes - cached_bytes + up <= mem_limit / 3) bytes = up;
+      const size_t up = (bytes + unit - 1) / unit * unit, live = held_bytes - cached_bytes;
+      size_t freeb = 0, total = 0;
+      if (up > bytes && (!mem_limit || live + up <= mem_limit / 16) &&
+          cudaMemGetInfo(&freeb, &total) == cudaSuccess && live + up <= freeb / 16)
+        bytes = up;
     }
     // make room: drop cached blocks before exceeding the budget
     while (mem_limit && held_bytes + bytes > mem_limit && !free_blocks.empty()) {
@@ -319,27 +329,35 @@ struct Engine {
     }
     if (mem_limit && held_bytes + bytes > mem_limit) return nullptr;
     void* p = nullptr;
-    if (cudaMallocAsync(&p, bytes, stream) != cudaSuccess) {
+    auto map = [&]() {
+      if (cudaMallocAsync(&p, bytes, stream) == cudaSuccess) return true;
       cudaGetLastError();
-      // the device itself is full (other contexts hold the rest): give the
-      // cached blocks back to the pool and try once more
-      if (free_blocks.empty()) return nullptr;
-      for (auto& fb : free_blocks) {
-        cudaFreeAsync(fb.second.p, stream);
-        held_bytes -= fb.first;
-      }
-      free_blocks.clear();
-      cached_bytes = 0;
-      if (cudaMallocAsync(&p, bytes, stream) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
+      return false;
+    };
+    if (!map()) {
+      // the device itself is full (others hold the rest): the size asked for,
+      // then give the cached blocks back to the pool and try once more
+      const bool rounded = bytes != asked;
+      bytes = asked;
+      if (!rounded || !map()) {
+        if (free_blocks.empty()) return nullptr;
+        drop_cache();
+        if (!map()) return nullptr;
       }
     }
     held_bytes += bytes;
     live_blocks[p] = bytes;
-    *got = bytes;
+    *got = asked;
     peak_live = std::max(peak_live, held_bytes - cached_bytes);
     return p;
+  }
+
+  // Every cached block back to the device's memory pool.
+  void drop_cache() {
+    for (auto& fb : free_blocks) cudaFreeAsync(fb.second.p, stream);
+    free_blocks.clear();
+    held_bytes -= cached_bytes;
+    cached_bytes = 0;
   }
 
   // After a call: keep cached at most what the call had live at its peak (the
@@ -1684,10 +1702,7 @@ struct Engine {
   // first, since the arena takes their memory.
   void open_arena() {
     if (arena.base) return;
-    for (auto& kv : free_blocks) cudaFreeAsync(kv.second.p, stream);
-    free_blocks.clear();
-    held_bytes -= cached_bytes;
-    cached_bytes = 0;
+    drop_cache();
     const size_t gran = (size_t)1 << 21;
     size_t want = mem_limit > held_bytes ? (mem_limit - held_bytes) & ~(gran - 1) : 0;
     size_t least = (size_t)1 << 30;
