@@ -20,6 +20,7 @@
 #include <cstring>
 #include <deque>
 #include <map>
+#include <mutex>
 #include <new>
 #include <functional>
 #include <vector>
@@ -200,6 +201,44 @@ struct Engine {
 
   ~Engine() { release(); }
 
+  // The engines of the process.  A call holds its engine's mutex; an engine
+  // whose allocation finds the device full takes what the idle ones (in no
+  // call) keep cached.
+  std::mutex in_call;
+  struct Registry {
+    std::mutex mu;
+    std::vector<Engine*> all;
+  };
+  static Registry& registry() {
+    static Registry* r = new Registry;   // (never destroyed: engines may end after static objects)
+    return *r;
+  }
+  // f(engine) for every idle engine of device dev but `self`, under its mutex.
+  // (Only try_lock inside: a call that holds its own mutex waits for nobody's.)
+  template <typename F>
+  static void each_idle(int dev, const Engine* self, F&& f) {
+    Registry& r = registry();
+    std::lock_guard<std::mutex> g(r.mu);
+    for (Engine* e : r.all) {
+      if (e == self || e->device != dev || !e->in_call.try_lock()) continue;
+      f(*e);
+      e->in_call.unlock();
+    }
+  }
+  // The idle engines' cached blocks back to the device; false: there were none.
+  bool reclaim_idle() {
+    bool any = false;
+    each_idle(device, this, [&](Engine& e) {
+      if (e.free_blocks.empty()) return;
+      e.drop_cache();
+      cudaStreamSynchronize(e.stream);
+      any = true;
+    });
+    cudaMemPool_t pool;
+    if (any && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    return any;
+  }
+
   // Records (and with VFB_DEBUG=1 prints) the CUDA error behind a failure.
   vfb_status dev_fail(int line) {
     const cudaError_t e = cudaGetLastError();
@@ -336,13 +375,14 @@ struct Engine {
     };
     if (!map()) {
       // the device itself is full (others hold the rest): the size asked for,
-      // then give the cached blocks back to the pool and try once more
+      // then with the cached blocks given back to the pool, then with those of
+      // the process's idle engines
       const bool rounded = bytes != asked;
       bytes = asked;
       if (!rounded || !map()) {
-        if (free_blocks.empty()) return nullptr;
+        const bool dropped = !free_blocks.empty();
         drop_cache();
-        if (!map()) return nullptr;
+        if (!(dropped && map()) && !(reclaim_idle() && map())) return nullptr;
       }
     }
     held_bytes += bytes;
@@ -363,7 +403,8 @@ struct Engine {
   // After a call: keep cached at most what the call had live at its peak (the
   // blocks the next call of its kind reuses), or an eighth of the budget where
   // that is more (calls in turn whose needs differ); the rest goes back to the
-  // device's memory pool, where other contexts of the process can allocate it.
+  // device's memory pool, where other contexts of the process can allocate it;
+  // what is kept, they take when they need it (reclaim_idle).
   // The blocks released longest ago go first: the call's final buffers,
   // released last, stay.  (Dropping the largest first, down to the call's peak,
   // made a solve whose rows are 0.4% larger than the last one's map 6 GB of
@@ -421,15 +462,17 @@ struct Engine {
     sms = prop.multiProcessorCount;
     size_t freeb = 0, total = 0;
     cudaMemGetInfo(&freeb, &total);
-    // memory the process's pool holds but has not handed out is available too
+    // memory the process's pool holds but has not handed out is available too,
+    // and what idle engines keep cached
     size_t pool_spare = 0;
+    each_idle(device, this, [&](Engine& e) { pool_spare += e.cached_bytes; });
     {
       cudaMemPool_t dp;
       uint64_t reserved = 0, used = 0;
       if (cudaDeviceGetDefaultMemPool(&dp, device) == cudaSuccess &&
           cudaMemPoolGetAttribute(dp, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
           cudaMemPoolGetAttribute(dp, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-        pool_spare = (size_t)(reserved - used);
+        pool_spare += (size_t)(reserved - used);
     }
     mem_limit = (o && o->mem_limit_bytes) ? o->mem_limit_bytes : (size_t)(0.9 * (double)(freeb + pool_spare));
     if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return VFB_DEVICE_ERROR;
@@ -1716,10 +1759,15 @@ struct Engine {
       }
     }
     void* p = nullptr;
+    bool alone = false;   // idle engines' caches taken
     while (want >= least && want > 0) {
       if (cudaMallocAsync(&p, want, stream) == cudaSuccess) break;
       cudaGetLastError();
       p = nullptr;
+      if (!alone) {
+        alone = true;
+        if (reclaim_idle()) continue;
+      }
       want = (want / 2) & ~(gran - 1);
     }
     if (!p || cudaStreamSynchronize(stream) != cudaSuccess) {
@@ -2622,14 +2670,27 @@ vfb_status vfb_create(void** ctx, const vfb_opts* opts) {
     delete e;
     return s;
   }
+  Engine::Registry& r = Engine::registry();
+  std::lock_guard<std::mutex> g(r.mu);
+  r.all.push_back(e);
   *ctx = e;
   return VFB_OK;
 }
 
-void vfb_destroy(void* ctx) { delete static_cast<Engine*>(ctx); }
+void vfb_destroy(void* ctx) {
+  if (!ctx) return;
+  Engine* e = static_cast<Engine*>(ctx);
+  {
+    Engine::Registry& r = Engine::registry();
+    std::lock_guard<std::mutex> g(r.mu);
+    r.all.erase(std::remove(r.all.begin(), r.all.end(), e), r.all.end());
+  }
+  delete e;
+}
 
 vfb_status vfb_solve(void* ctx, const vfb_instance* inst, vfb_result* out) {
   if (!ctx || !inst || !out) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   const vfb_status rc = static_cast<Engine*>(ctx)->batch(inst, 1, out);
   return rc != VFB_OK ? rc : out->status;
 }
@@ -2639,6 +2700,7 @@ vfb_status vfb_solve_costs(void* ctx, const vfb_instance* inst, const int* costs
   if (neg_type != 1 && neg_type != 2) return VFB_BAD_INPUT;
   for (int c = 0; c < 8; ++c)
     if (costs[c] < 1 || costs[c] > VFB_MAX_SIZE) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   Engine* e = static_cast<Engine*>(ctx);
   for (int c = 0; c < 8; ++c) e->req_cost[c] = costs[c];
   e->req_neg = neg_type;
@@ -2651,6 +2713,7 @@ vfb_status vfb_solve_costs(void* ctx, const vfb_instance* inst, const int* costs
 vfb_status vfb_solve_bs(void* ctx, const vfb_instance* inst, int bs_max_size, vfb_result* out) {
   if (!ctx || !inst || !out) return VFB_BAD_INPUT;
   if (bs_max_size < 1 || bs_max_size > VFB_MAX_SIZE) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   Engine* e = static_cast<Engine*>(ctx);
   e->bs_max = bs_max_size;
   const vfb_status rc = e->batch(inst, 1, out);
@@ -2660,16 +2723,19 @@ vfb_status vfb_solve_bs(void* ctx, const vfb_instance* inst, int bs_max_size, vf
 
 vfb_status vfb_solve_exhaustive(void* ctx, const vfb_instance* inst, vfb_result* out) {
   if (!ctx || !inst || !out) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   return static_cast<Engine*>(ctx)->exhaustive(*inst, *out);
 }
 
 vfb_status vfb_batch_solve(void* ctx, const vfb_instance* inst, int n, vfb_result* out) {
   if (!ctx || (n > 0 && (!inst || !out)) || n < 0) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   return static_cast<Engine*>(ctx)->batch(inst, n, out);
 }
 
 vfb_status vfb_serve_open(void* ctx, int slots, int max_traces) {
   if (!ctx) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   return static_cast<Engine*>(ctx)->serve_open(slots, max_traces);
 }
 
@@ -2685,11 +2751,14 @@ vfb_status vfb_serve_submit(void* ctx, const vfb_instance* inst, uint64_t tag) {
 
 vfb_status vfb_serve_step(void* ctx, vfb_served* done, int cap, int* ndone, int* active, int* queued) {
   if (!ctx || !done || !ndone || cap <= 0) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   return static_cast<Engine*>(ctx)->serve_step(done, cap, ndone, active, queued);
 }
 
 void vfb_serve_close(void* ctx) {
-  if (ctx) static_cast<Engine*>(ctx)->serve_close();
+  if (!ctx) return;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
+  static_cast<Engine*>(ctx)->serve_close();
 }
 
 vfb_status vfb_tune_set(void* ctx, const vfb_tune* tune) {
@@ -2705,6 +2774,7 @@ vfb_status vfb_tune_get(void* ctx, vfb_tune* tune) {
 
 vfb_status vfb_autotune(void* ctx, const vfb_instance* sample, int n, int reps, vfb_tune* out) {
   if (!ctx) return VFB_BAD_INPUT;
+  std::lock_guard<std::mutex> in_call(static_cast<Engine*>(ctx)->in_call);
   return static_cast<Engine*>(ctx)->autotune(sample, n, reps, out);
 }
 
