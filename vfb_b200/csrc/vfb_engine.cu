@@ -1671,6 +1671,7 @@ struct Engine {
     std::vector<uint64_t> words;
     std::vector<int> lengths;
     bool evicted = false;   // gave its slot up for memory: waits until no request waits
+    vfb_status refused = VFB_OK;   // its upload failed: to be reported with this status
   };
   struct Session {
     int cap = 0;
@@ -1846,6 +1847,14 @@ struct Engine {
     }
   }
 
+  // A request to the head of the queue (its arrays move with it).
+  void requeue(Pending&& p) {
+    sv.queue.push_front(std::move(p));
+    Pending& q = sv.queue.front();
+    q.in.words = q.words.data();
+    q.in.lengths = q.lengths.data();
+  }
+
   vfb_status serve_step(vfb_served* done, int cap_done, int* ndone, int* active, int* queued) {
     *ndone = 0;
     if (sv.cap <= 0) return VFB_BAD_INPUT;
@@ -1867,10 +1876,10 @@ struct Engine {
       Pending& p = sv.queue.front();
       // an evicted request comes back once no request waits for memory
       // (else it would take memory the waiting ones need and be evicted again)
-      if (p.evicted && sv.pressure && nbusy > 0) break;
+      if (p.refused == VFB_OK && p.evicted && sv.pressure && nbusy > 0) break;
       InstHost& H = sv.H[i];
       H = InstHost{};
-      vfb_status s = prepare(p.in, H);
+      vfb_status s = p.refused != VFB_OK ? p.refused : prepare(p.in, H);
       const int tp = p.in.num_traces + (p.in.num_traces & 1);
       if (s == VFB_OK && tp > sv.tp) s = VFB_LIMIT;
       if (s == VFB_OK) {
@@ -1900,14 +1909,15 @@ struct Engine {
         H.d.p1_quota = sv.step_cands;
       }
       if (s != VFB_OK) {
-        // refused: report it as finished with that status
+        // refused: report it as finished with that status (in a later step
+        // when done[] is full: it stays at the head of the queue)
         if (H.d.rows) free_buffers(H);
-        if (*ndone < cap_done) {
-          std::memset(&done[*ndone], 0, sizeof(vfb_served));
-          done[*ndone].tag = p.tag;
-          done[*ndone].result.status = s;
-          ++*ndone;
-        }
+        H = InstHost{};
+        if (*ndone >= cap_done) break;
+        std::memset(&done[*ndone], 0, sizeof(vfb_served));
+        done[*ndone].tag = p.tag;
+        done[*ndone].result.status = s;
+        ++*ndone;
         sv.queue.pop_front();
         continue;
       }
@@ -1939,17 +1949,16 @@ struct Engine {
         c_h2d += sizeof(InstDev);
       }
       if (s != VFB_OK) {
-        // refused: reported as finished with that status, as above
-        for (int i : admitted) {
+        // none of them started: back to the head of the queue in their order,
+        // from where the next steps report them, as many as done[] holds
+        for (size_t j = admitted.size(); j-- > 0;) {
+          const int i = admitted[j];
           cudaMemsetAsync(&dInst[i].status, 0, sizeof(int), stream);   // (ST_IDLE)
           free_buffers(sv.H[i]);
           sv.H[i] = InstHost{};
           sv.busy[i] = 0;
-          if (*ndone >= cap_done) continue;
-          std::memset(&done[*ndone], 0, sizeof(vfb_served));
-          done[*ndone].tag = sv.tag[i];
-          done[*ndone].result.status = s;
-          ++*ndone;
+          requeue(std::move(sv.req[i]));
+          sv.queue.front().refused = s;
         }
       } else {
         k_fill<<<grid, 256, 0, stream>>>(hB);
@@ -2043,10 +2052,8 @@ struct Engine {
         sv.H[v] = InstHost{};
         sv.busy[v] = 0;
         for (int i : waiting) sv.waited[i] = 0;
-        sv.req[v].evicted = true;
-        sv.queue.push_front(std::move(sv.req[v]));
-        sv.queue.front().in.words = sv.queue.front().words.data();
-        sv.queue.front().in.lengths = sv.queue.front().lengths.data();
+        requeue(std::move(sv.req[v]));
+        sv.queue.front().evicted = true;
         const int idle = ST_IDLE;
         cudaMemcpyAsync(&dInst[v].status, &idle, sizeof(int), cudaMemcpyHostToDevice, stream);
         ++sv.evictions;
