@@ -13,13 +13,13 @@ namespace vfb {
 
 constexpr int kMaxTraces = 128;
 constexpr int kMaxSize = 32;          // formula size limit (ltl_nocache.cu:11)
-constexpr int kMaxSplits = 16;        // floor((32-1)/2)
 // P1 operand groups of a level: up to 4 unary (one per operand level) and the
 // binary level pairs; with unit costs, 1 + floor((k-1)/2)
 constexpr int kGroups = 64;
 constexpr int kTS = 128;              // stream rows per P1 tile (= threads per CTA)
 // Staged rows per P1 tile (maximum).  Only the staged rows are held in shared
-// memory (32 bytes per word, see QWord): 16 rows of 64 words are 32 KB.
+// memory (32 bytes per word, see QWord): 16 rows of up to 16 words, 8, 4 or 2
+// of longer ones (p1_rows_max), 264 words at most.
 constexpr int kTQ = 16;
 constexpr int kTQDefault = 16;        // staged rows per P1 tile unless the tune table says otherwise
 constexpr int kP1TileTarget = 4096;   // shrink the staged height until a level has this many tiles

@@ -61,6 +61,7 @@ uint64_t pow2_at_most(uint64_t x) {
 
 // Kernels of one level step, in launch order (ids index Engine::prof).
 enum KId { KP_ADVANCE, KP_P1, KP_TSCAN, KP_COMPACT, KP_EMIT, KP_INIT, KP_REHASH, KP_N };
+// (labels of the profile; "k_table_scan" is k_table_scan_check)
 const char* const kNames[KP_N] = {"k_advance", "k_p1", "k_table_scan", "k_compact", "k_emit", "k_init",
                                   "k_rehash"};
 // One launch of the step graph: plan the instances that need it, then build
@@ -115,7 +116,7 @@ struct Engine {
   // batch workspace
   int ninst_cap = 0;
   BatchDev hB{};
-  BatchDev* dB = nullptr;
+  BatchDev* dB = nullptr;     // hB on the device, for the cooperative solver (the others take it by value)
   InstDev* dInst = nullptr;
   int2* h_status = nullptr;   // pinned mirror of B.status_out
   unsigned int* h_ctl = nullptr;  // pinned mirror of B.ctl, then of B.loop_iter

@@ -10,14 +10,18 @@
 //                 whose CS satisfies the sample is recorded
 //                 (applyOperator LTL_BS.cu:183-238, makeRlxUnqChkCSs 30-110,
 //                  processUniqueCS 251-269)
-//   k_table_scan  a slot whose final payload carries level k holds a key first
+//   k_table_scan_check
+//                 a slot whose final payload carries level k holds a key first
 //                 seen at this level; its payload's index is the key's owner
 //                 (the minimum candidate index): set the owner's bit.  Also
 //                 settles whether the recorded solution candidate owns its key
+//                 and checks the level's buffers; of a few instances' small
+//                 levels it compacts the bitmap too
 //   k_compact     ordered compaction of the owner bitmap into the ascending
-//                 owner list and the owners' rows appended to the level cache
-//                 in canonical order, solution test (insertInCache
-//                 LTL_BS.cu:299-329); rows skipped when the solution is settled
+//                 owner list
+//   k_emit        the owners' rows appended to the level cache in canonical
+//                 order, solution test (insertInCache LTL_BS.cu:299-329); rows
+//                 skipped when the solution is settled
 //   k_advance     level bookkeeping, formula reconstruction (LTL_BS.cu:561-705),
 //                 then the next level's candidate-block bases, P1 tiling and
 //                 buffer checks (LTL_BS.cu:1226-1488)
@@ -123,23 +127,25 @@ __device__ void plan_one(InstDev& I, bool few) {
   // operand groups: the unary operators by operand level (bits ~ X F G), the
   // binary ones by level pair la <= lb (bits &, |, la U lb, lb U la); with
   // unit costs one unary group and one group per split, as the reference's
-  // launches fuse them.  The tiles of every staged height 2^0..2^5 are summed
-  // on the way.
+  // launches fuse them.  The tiles of every staged height 2^0..2^4 (kTQ) are
+  // summed on the way.
   int ng = 0;
-  uint64_t tl[6] = {0, 0, 0, 0, 0, 0}, tsplit = 0;   // (tsplit: kTS/4 rows a tile, one staged)
+  constexpr int kHeights = 5;
+  static_assert(1 << (kHeights - 1) == kTQ, "");
+  uint64_t tl[kHeights] = {0, 0, 0, 0, 0}, tsplit = 0;   // (tsplit: kTS/4 rows a tile, one staged)
   auto add_tiles = [&](int kind, int la, int lb) {
     if (kind == 0) {
       const uint64_t st = (n[la] + kTS - 1) / kTS;
       tsplit += (n[la] + kTS / 4 - 1) / (kTS / 4);
 #pragma unroll
-      for (int u = 0; u < 6; ++u) tl[u] += (st + (1ULL << u) - 1) >> u;
+      for (int u = 0; u < kHeights; ++u) tl[u] += (st + (1ULL << u) - 1) >> u;
     } else {
       const bool qleft = (la == lb) || (n[la] <= n[lb]);
       const uint64_t nS = qleft ? n[lb] : n[la], nQ = qleft ? n[la] : n[lb];
       const uint64_t st = (nS + kTS - 1) / kTS;
       tsplit += (nS + kTS / 4 - 1) / (kTS / 4) * nQ;
 #pragma unroll
-      for (int u = 0; u < 6; ++u) tl[u] += st * ((nQ + (1ULL << u) - 1) >> u);
+      for (int u = 0; u < kHeights; ++u) tl[u] += st * ((nQ + (1ULL << u) - 1) >> u);
     }
   };
   // unit costs: one group per size split, then one unary group over level
@@ -236,7 +242,7 @@ __device__ void plan_one(InstDev& I, bool few) {
   int lg = 0;
   uint64_t t = tl[0];
 #pragma unroll
-  for (int u = 1; u < 6; ++u)
+  for (int u = 1; u < kHeights; ++u)
     if ((1 << u) <= rows_cap && tl[u] >= target) { lg = u; t = tl[u]; }
   I.tq = 1 << lg;
   // four lanes to a stream row where the level then still runs in one wave
@@ -706,6 +712,7 @@ __global__ void __launch_bounds__(kTS, 4) k_p1(const __grid_constant__ BatchDev 
 // level k.  One chunk of scan_slots slots per CTA iteration; an empty slot's
 // payload (~0) carries no level <= 32.  One warp per instance also settles
 // whether the recorded solution candidate owns its key.
+
 // The table scan's counting mode at a level that has a solution candidate
 // after P1.  The fields read are not written during the scan, except no_mask:
 // a failed ownership check sets it while other CTAs of a batch still scan the
@@ -888,7 +895,10 @@ __device__ void ph_table_scan(const BatchDev& B, unsigned bid, unsigned nb) {
 // shortfall asks the host for memory before anything of the level is
 // written), its row-emission items.  The owners are known after the level's
 // last slice of P1 tiles; an earlier slice (n_wins still 0) only stops at a
-// failed probe.
+// failed probe.  A counted last level (last_unsolved) needs neither list nor
+// rows, and is held to the same buffers all the same: which searches a budget,
+// a request's cap or the static scratch holds stays what it is for a level
+// that is written.
 __device__ unsigned long long check_level(InstDev& I) {
   // (status, sol_known and n_wins may have been changed by this kernel: from the L2)
   const int status = __ldcg(&I.status), sk = __ldcg(&I.sol_known), k = ld_now(I.level);
@@ -1518,9 +1528,9 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(const __grid_consta
 // ================================================================ row emission
 // Graph solver: the owners' rows appended to the level cache in canonical
 // order, solution test (insertInCache LTL_BS.cu:299-329).  Work items are
-// kEmitItem consecutive owners of one instance on large levels, kEmitGroup
-// on small ones (prefix built by k_table_scan_check, which records the
-// choice).  A warp takes an item: each lane decodes one owner (decode_level:
+// kEmitGroup consecutive owners of one instance on small levels, doubled up to
+// kEmitItem on larger ones (prefix built by k_table_scan_check, which records
+// the choice).  A warp takes an item: each lane decodes one owner (decode_level:
 // compares with the plan's block bases); the item's rows are one block of the
 // level cache, which the lanes write 16 bytes at a time side by side, whatever
 // the rows' pitch, kEmitUnroll pieces of their operand rows in flight.

@@ -17,7 +17,7 @@ constexpr int kCompactThreads = 256;  // threads per k_compact CTA (two bitmap w
 constexpr int kAdvanceThreads = 256;
 constexpr int kTickets = 8;            // words of BatchDev::tickets
 constexpr int kTicketP1Blocks = 4;     // tickets[4]: CTAs the step's k_p1 runs (0: all), set by k_advance
-constexpr int kEmitGroup = 4;         // owners per warp step of k_emit (their loads in flight together)
+constexpr int kEmitGroup = 4;         // owners per k_emit work item at least (doubled as the level grows)
 constexpr int kEmitItem = 32;         // owners per k_emit work item at most (one warp; a lane
                                       // decodes each); small levels take as few as kEmitGroup so
                                       // that their owners still spread over many warps

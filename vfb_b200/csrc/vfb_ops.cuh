@@ -353,20 +353,6 @@ __device__ __forceinline__ const uint64_t* row_ptr(const InstDev& I, int lvl, ui
   return I.rows + (I.lstart[lvl] + idx) * (uint64_t)I.TP;
 }
 
-template <int MODE>
-__device__ inline void cand_key(const InstDev& I, const Cand& c, uint64_t& h, uint64_t& l) {
-  const uint64_t* ra = row_ptr(I, c.la, c.a);
-  const uint64_t* rb = (c.op == OP_AND || c.op == OP_OR || c.op == OP_U) ? row_ptr(I, c.lb, c.b) : ra;
-  KeyAcc k;
-  key_init(k);
-  const int T = I.T, half = T / 2;
-  for (int t = 0; t < T; ++t) {
-    const uint64_t w = apply_w(c.op, ra[t], rb[t], I.len[t]);
-    key_word<MODE>(k, w, t, half, I.off[t], I.width[t], I.stride1, I.len[t]);
-  }
-  key_final<MODE>(k, h, l);
-}
-
 // ======================================================================= P1
 // Shared per-tile parameters.  s: the stream operand (a row per thread), q:
 // the staged operand (up to kTQ rows, read by every thread).
@@ -802,8 +788,8 @@ __device__ __forceinline__ void take_pair(const TileSh& P, uint64_t q, uint64_t 
 }
 
 // Hash keys.  Bound by instruction issue and the ALU pipe (level 8 of the large
-// instance: 5.5 M candidates of 63 words in 0.61 ms, before 1.09 ms; ALU pipe
-// 62%): per word, 11 ALU instructions for & or |, 16 for a U, and 6 multiplies
+// instance: 5.5 M candidates of 63 words in 0.623 ms, before 1.092 ms; ALU pipe
+// 65%): per word, 11 ALU instructions for & or |, 16 for a U, and 6 multiplies
 // each.  The first xor-shift of a & b is (a & b) ^ (a >> 30 & b >> 30), so the
 // shifted words are made once per row and word, and the reversed words of U
 // too; the last xor-shift is taken once per key (splitmix_end).
