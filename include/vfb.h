@@ -56,7 +56,7 @@ typedef struct {
   int device;              /* CUDA device ordinal */
   size_t mem_limit_bytes;  /* device memory budget of one solve/batch (0: 90% of the memory
                               free at creation, counting what the process's stream-ordered
-                              pool holds unused) */
+                              pool holds unused and its idle contexts keep cached) */
   int verbose;             /* 1: per-level progress lines on stderr */
   int profile;             /* 1: time every kernel of the level step with CUDA events
                               (see vfb_profile_read); adds one event pair per kernel */
@@ -64,7 +64,9 @@ typedef struct {
 
 /* One learning problem.  Layout as ltl_nocache's readJsonFile: words[i*num_vars + v]
  * holds proposition v on trace i (bit t = value at step t); traces 0..num_pos-1
- * are positive, the rest negative; lengths[i] is trace i's length (1..64). */
+ * are positive, the rest negative; lengths[i] is trace i's length (1..64).  Bits
+ * at and past the length should be 0: the operators work on whole words, so F, G
+ * and U see them. */
 typedef struct {
   int num_vars;
   int num_traces;
@@ -199,7 +201,8 @@ vfb_status vfb_solve_noalloc(const vfb_instance *inst, vfb_result *out);
  * allocation, halved until it can be had, and the session's buffers are
  * carved out of it, so that growth inside a step maps no new device memory;
  * vfb_serve_close gives it back to the engine's pool (vfb_destroy returns
- * the pool's memory to the device). */
+ * the pool's memory to the device).  done[] holds cap results; what a step has
+ * beyond them (refused requests too) comes with later steps. */
 typedef struct {
   uint64_t tag;
   vfb_result result;
